@@ -93,6 +93,8 @@ struct SdfBatchLaunch {
     int totalTris;
     long long totalQuads;
     int constructThreads;
+    TriJob* jobs;         // [totalTris]: written by the initialisation, read by the construct; null when the
+                          // construct makes its own (sdf_takes_jobs)
     int expand;      // some SDF keeps a corner-expanded copy: run the expansion
     // the SDFs that keep one, so that the expansion runs over their cells only: their indices into
     // `sdfs`, the prefix of their cell counts (nexp + 1 entries), and the sum

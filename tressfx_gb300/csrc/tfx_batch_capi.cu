@@ -91,6 +91,7 @@ struct tfx_batch_t {
     SdfBatchLaunch sdfL{};
     SdfTileLaunch sdfT{};           // the tiled construct's tables
     void* tileArena = nullptr;
+    void* jobArena = nullptr;       // SdfBatchLaunch::jobs
     int sdfForm = 0;                // TFX_BATCH_SDF_FORM: 0 one warp per triangle, 1 tiles (when the grids allow)
     bool tilesAvailable = false;
 
@@ -177,6 +178,7 @@ extern "C" int tfx_batch_destroy(tfx_batch b) {
     if (b->expandedArena) cudaFree(b->expandedArena);
     if (b->expTable) cudaFree(b->expTable);
     if (b->tileArena) cudaFree(b->tileArena);
+    if (b->jobArena) cudaFree(b->jobArena);
     for (auto t : b->levelPairs)
         if (t) cudaFree(t);
     for (auto& c : b->classes)
@@ -874,7 +876,10 @@ extern "C" int tfx_batch_build(tfx_batch b, int reserved) {
     }
     if (nsdf > 0)
         TFX_CUDA(cudaMemcpy(b->sdfTable, sdfs.data(), sizeof(BatchSdf) * nsdf, cudaMemcpyHostToDevice), "tfx_batch: SDFs");
-    b->sdfL = SdfBatchLaunch{b->sdfTable, nsdf, firstTri, firstQuad, 128, 0, nullptr, nullptr, 0, 0};
+    if (sdf_takes_jobs(firstTri))
+        TFX_CUDA(cudaMalloc(&b->jobArena, sdf_job_bytes() * (size_t)firstTri), "tfx_batch: triangle jobs");
+    b->sdfL = SdfBatchLaunch{b->sdfTable, nsdf, firstTri, firstQuad, 128, reinterpret_cast<TriJob*>(b->jobArena),
+                             0, nullptr, nullptr, 0, 0};
     b->expandMode = 2;
     if (int r = apply_expand_mode(b)) return r;
 

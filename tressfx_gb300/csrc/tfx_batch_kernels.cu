@@ -79,11 +79,24 @@ __device__ __forceinline__ int find_by_prefix_quad(const BatchSdf* __restrict__ 
     return lo;
 }
 
+// The job of triangle t of the batch's triangle list (which spans the SDFs).
+__device__ __forceinline__ TriJob batch_job(const BatchSdf* __restrict__ sdfs, int nsdf, int t) {
+    const BatchSdf& s = sdfs[find_by_prefix_tri(sdfs, nsdf, t)];
+    const size_t tri = (size_t)(t - s.firstTriangle);
+    const float3 x0 = xyz(__ldg(s.mesh + 2 * (size_t)__ldg(s.indices + 3 * tri + 0)));
+    const float3 x1 = xyz(__ldg(s.mesh + 2 * (size_t)__ldg(s.indices + 3 * tri + 1)));
+    const float3 x2 = xyz(__ldg(s.mesh + 2 * (size_t)__ldg(s.indices + 3 * tri + 2)));
+    return tri_job(s.frame->grid, s.words, x0, x1, x2);
+}
+
 // InitializeSignedDistanceField, :301-312: every cell of every SDF, 4 cells per thread (the last
-// quad of an SDF may be partial).
-__global__ void __launch_bounds__(256) k_batch_sdf_init(const BatchSdf* __restrict__ sdfs, int nsdf, long long totalQuads) {
+// quad of an SDF may be partial), and with a job array the job of every triangle.
+__global__ void __launch_bounds__(256) k_batch_sdf_init(const BatchSdf* __restrict__ sdfs, int nsdf, long long totalQuads,
+                                                        TriJob* __restrict__ jobs, int totalTris) {
     const uint32_t v = float_flip3(1e10f);
     const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < totalTris; t += stride)
+        jobs[t] = batch_job(sdfs, nsdf, (int)t);
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < totalQuads; q += stride) {
         const BatchSdf& s = sdfs[find_by_prefix_quad(sdfs, nsdf, q)];
         const long long c = 4 * (q - s.firstQuad);
@@ -148,26 +161,28 @@ __global__ void __launch_bounds__(256) k_batch_sdf_expand(const BatchSdf* __rest
     }
 }
 
-// ConstructSignedDistanceField, :329-397.  Each warp takes chunks of `per` (<= 32) consecutive
-// triangles of the batch's triangle list (which may span SDFs): lane k finds the SDF of the chunk's
-// k-th triangle and makes its job, then the warp runs the triangles' cell loops in turn.
-// WARPS = warps per block; STAGED as in sdf_construct_chunk_warp.
-template <int WARPS, bool STAGED>
-__global__ void __launch_bounds__(WARPS * 32) k_batch_sdf_construct(const BatchSdf* __restrict__ sdfs, int nsdf,
-                                                                     int totalTris, int per) {
-    __shared__ TriJob jobs[STAGED ? WARPS : 1][STAGED ? kTriJobsPerWarp : 1];
+// ConstructSignedDistanceField, :329-397, over the jobs k_batch_sdf_init made (every SDF's triangles in
+// one list).  WARPS = warps per block.
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? kConstructBlocksPerSM : 1) k_batch_sdf_construct(const TriJob* __restrict__ jobs, int totalTris) {
+    extern __shared__ __align__(16) unsigned char smem_sdf[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const SdfWarpArea area = sdf_warp_area(smem_sdf, warp, kSdfJobsAhead);
+    sdf_construct_jobs_warp(area, jobs, totalTris, blockIdx.x * WARPS + warp, gridDim.x * WARPS, lane);
+}
+
+// The same without a job array (small batches): each warp takes chunks of `per` consecutive triangles,
+// lane k making the job of the chunk's k-th.
+__global__ void __launch_bounds__(128) k_batch_sdf_construct_chunks(const BatchSdf* __restrict__ sdfs, int nsdf, int totalTris,
+                                                                    int per) {
+    extern __shared__ __align__(16) unsigned char smem_sdf[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const SdfWarpArea area = sdf_warp_area(smem_sdf, warp, per);
     const int chunks = (totalTris + per - 1) / per;
-    for (int k = blockIdx.x * WARPS + warp; k < chunks; k += gridDim.x * WARPS) {
+    for (int k = blockIdx.x * 4 + warp; k < chunks; k += gridDim.x * 4) {
         const int first = k * per;
-        sdf_construct_chunk_warp<STAGED>(jobs[STAGED ? warp : 0], first, min(per, totalTris - first), lane, [&](int t) {
-            const BatchSdf& s = sdfs[find_by_prefix_tri(sdfs, nsdf, t)];
-            const int tri = t - s.firstTriangle;
-            const float3 x0 = xyz(__ldg(s.mesh + 2 * (size_t)__ldg(s.indices + 3 * tri + 0)));
-            const float3 x1 = xyz(__ldg(s.mesh + 2 * (size_t)__ldg(s.indices + 3 * tri + 1)));
-            const float3 x2 = xyz(__ldg(s.mesh + 2 * (size_t)__ldg(s.indices + 3 * tri + 2)));
-            return tri_job(s.frame->grid, s.words, x0, x1, x2);
-        });
+        sdf_construct_chunk_warp(area, first, min(per, totalTris - first), lane,
+                                 [&](int t) { return batch_job(sdfs, nsdf, t); });
     }
 }
 
@@ -1240,30 +1255,35 @@ cudaError_t launch_collide_level(const BatchObject* objs, const BatchSdf* sdfs, 
     return cudaGetLastError();
 }
 
+static int sdf_construct_blocks_per_sm(int threads) {
+    int nb = 0;
+    const size_t smem = sdf_construct_smem(threads / 32, kSdfJobsAhead);
+    const cudaError_t e = threads == 64    ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_batch_sdf_construct<2>, 64, smem)
+                          : threads == 256 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_batch_sdf_construct<8>, 256, smem)
+                                           : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_batch_sdf_construct<4>, 128, smem);
+    return e == cudaSuccess && nb > 0 ? nb : 1;
+}
+
 cudaError_t launch_batch_sdf(const SdfBatchLaunch& L, cudaStream_t s) {
     if (L.nsdf <= 0) return cudaSuccess;
     const long long q = L.totalQuads;
     const unsigned gq = (unsigned)std::min<long long>((q + 255) / 256, (long long)sm_count() * 32);
-    k_batch_sdf_init<<<gq, 256, 0, s>>>(L.sdfs, L.nsdf, q);
-    if (L.totalTris > 0) {
-        const int warpsPerBlock = L.constructThreads / 32;
+    const long long initWork = std::max<long long>(q, L.jobs ? L.totalTris : 0);
+    const unsigned gi = (unsigned)std::min<long long>((initWork + 255) / 256, (long long)sm_count() * 32);
+    k_batch_sdf_init<<<gi, 256, 0, s>>>(L.sdfs, L.nsdf, q, L.jobs, L.jobs ? L.totalTris : 0);
+    if (L.totalTris > 0 && L.jobs) {
+        const int wpb = L.constructThreads / 32;
+        const size_t smem = sdf_construct_smem(wpb, kSdfJobsAhead);
+        const unsigned blocks = (unsigned)std::min<long long>(((long long)L.totalTris + wpb - 1) / wpb,
+                                                              (long long)sm_count() * sdf_construct_blocks_per_sm(L.constructThreads));
+        if (wpb == 2) k_batch_sdf_construct<2><<<blocks, 64, smem, s>>>(L.jobs, L.totalTris);
+        else if (wpb == 8) k_batch_sdf_construct<8><<<blocks, 256, smem, s>>>(L.jobs, L.totalTris);
+        else k_batch_sdf_construct<4><<<blocks, 128, smem, s>>>(L.jobs, L.totalTris);
+    } else if (L.totalTris > 0) {
         const int per = sdf_construct_chunk(L.totalTris, sm_count());
         const long long chunks = ((long long)L.totalTris + per - 1) / per;
-        const unsigned blocks =
-            (unsigned)std::min<long long>((chunks + warpsPerBlock - 1) / warpsPerBlock, (long long)sm_count() * 64);
-        const bool staged = per >= kTriJobsStagedFrom;
-        if (warpsPerBlock == 2 && staged)
-            k_batch_sdf_construct<2, true><<<blocks, 64, 0, s>>>(L.sdfs, L.nsdf, L.totalTris, per);
-        else if (warpsPerBlock == 2)
-            k_batch_sdf_construct<2, false><<<blocks, 64, 0, s>>>(L.sdfs, L.nsdf, L.totalTris, per);
-        else if (warpsPerBlock == 8 && staged)
-            k_batch_sdf_construct<8, true><<<blocks, 256, 0, s>>>(L.sdfs, L.nsdf, L.totalTris, per);
-        else if (warpsPerBlock == 8)
-            k_batch_sdf_construct<8, false><<<blocks, 256, 0, s>>>(L.sdfs, L.nsdf, L.totalTris, per);
-        else if (staged)
-            k_batch_sdf_construct<4, true><<<blocks, 128, 0, s>>>(L.sdfs, L.nsdf, L.totalTris, per);
-        else
-            k_batch_sdf_construct<4, false><<<blocks, 128, 0, s>>>(L.sdfs, L.nsdf, L.totalTris, per);
+        const unsigned blocks = (unsigned)std::min<long long>((chunks + 3) / 4, (long long)sm_count() * 64);
+        k_batch_sdf_construct_chunks<<<blocks, 128, sdf_construct_smem(4, per), s>>>(L.sdfs, L.nsdf, L.totalTris, per);
     }
     k_batch_sdf_finalize<<<gq, 256, 0, s>>>(L.sdfs, L.nsdf, q);
     if (L.expand) return launch_batch_sdf_expand(L, s);

@@ -449,9 +449,31 @@ extern "C" int tfx_sdf_destroy(tfx_sdf s) {
     cudaSetDevice(s->ctx->device);
     cudaStreamSynchronize(s->ctx->stream);
     cudaFree(s->grid);
+    for (void* p : s->jobArrays) cudaFree(p);
     context_release(s->ctx);
     delete s;
     return TFX_OK;
+}
+
+// Makes the construct's job array hold `ntri` triangles.  An array that cannot be had is left out (the
+// construct then makes its jobs in shared memory, with the same result), so this never fails a call, and
+// a capture in progress on this thread is left alone (the array is not part of it).  A recorded frame
+// keeps the address it was recorded with, so a smaller array is kept until the SDF goes; each is at least
+// twice the one before.
+static void reserve_jobs(tfx_sdf s, int ntri) {
+    if (ntri <= s->jobsCap || cudaSetDevice(s->ctx->device) != cudaSuccess || !sdf_takes_jobs(ntri)) return;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) { cudaGetLastError(); return; }
+    const int64_t cap = std::max<int64_t>(ntri, 2 * s->jobsCap);
+    void* p = nullptr;
+    if (cudaMalloc(&p, sdf_job_bytes() * (size_t)cap) == cudaSuccess) {
+        s->jobArrays.push_back(p);
+        s->jobs = static_cast<TriJob*>(p);
+        s->jobsCap = cap;
+    } else {
+        cudaGetLastError();
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
 }
 
 extern "C" int tfx_sdf_set_mesh(tfx_sdf s, const void* mesh, int nverts, const uint32_t* idx, int ntri) {
@@ -459,6 +481,7 @@ extern "C" int tfx_sdf_set_mesh(tfx_sdf s, const void* mesh, int nverts, const u
         return fail(TFX_ERR_INVALID_ARGUMENT, "tfx_sdf_set_mesh: bad argument");
     if (((uintptr_t)mesh & 15) != 0) return fail(TFX_ERR_INVALID_ARGUMENT, "tfx_sdf_set_mesh: mesh buffer not 16-byte aligned");
     s->mesh = (const float4*)mesh; s->nverts = nverts; s->idx = idx; s->ntri = ntri;
+    reserve_jobs(s, ntri);
     return TFX_OK;
 }
 
@@ -480,7 +503,12 @@ static int sdf_kernel(tfx_sdf s, int kernel, const SdfGrid& g) {
         case TFX_KERNEL_SDF_INITIALIZE: e = launch_sdf_initialize(s->grid, cells, s->ctx->stream); break;
         case TFX_KERNEL_SDF_CONSTRUCT:
             if (s->ntri > 0 && !s->mesh) return fail(TFX_ERR_INVALID_ARGUMENT, "tfx_sdf: no collision mesh bound");
-            e = launch_sdf_construct(s->grid, g, s->mesh, s->idx, s->ntri, s->ctx->stream);
+            if (s->ntri <= s->jobsCap && sdf_takes_jobs(s->ntri)) {
+                e = launch_sdf_jobs(s->jobs, s->grid, g, s->mesh, s->idx, s->ntri, s->ctx->stream);
+                if (e == cudaSuccess) e = launch_sdf_construct_jobs(s->jobs, s->ntri, s->ctx->stream);
+            } else {
+                e = launch_sdf_construct(s->grid, g, s->mesh, s->idx, s->ntri, s->ctx->stream);
+            }
             break;
         case TFX_KERNEL_SDF_FINALIZE: e = launch_sdf_finalize(s->grid, cells, s->ctx->stream); break;
         default: return fail(TFX_ERR_INVALID_ARGUMENT, "tfx_sdf_dispatch: kernel %d is not an SDF build kernel", kernel);
@@ -500,8 +528,15 @@ extern "C" int tfx_sdf_update(tfx_sdf s, const tfx_sdf_grid* grid) {
     SdfGrid g;
     if (int r = check_grid(s, grid, &g, "tfx_sdf_update")) return r;
     TFX_CUDA(cudaSetDevice(s->ctx->device), "cudaSetDevice");
-    if (int r = sdf_kernel(s, TFX_KERNEL_SDF_INITIALIZE, g)) return r;
-    if (int r = sdf_kernel(s, TFX_KERNEL_SDF_CONSTRUCT, g)) return r;
+    if (s->ntri > 0 && s->mesh && s->ntri <= s->jobsCap && sdf_takes_jobs(s->ntri)) {   // the initialisation makes the jobs too
+        cudaError_t e = launch_sdf_initialize(s->grid, (int64_t)g.nx * g.ny * g.nz, s->ctx->stream, &g, s->mesh, s->idx, s->ntri,
+                                              s->jobs);
+        if (e == cudaSuccess) e = launch_sdf_construct_jobs(s->jobs, s->ntri, s->ctx->stream);
+        if (e != cudaSuccess) return cuda_fail(e, "SDF kernel launch");
+    } else {
+        if (int r = sdf_kernel(s, TFX_KERNEL_SDF_INITIALIZE, g)) return r;
+        if (int r = sdf_kernel(s, TFX_KERNEL_SDF_CONSTRUCT, g)) return r;
+    }
     return sdf_kernel(s, TFX_KERNEL_SDF_FINALIZE, g);
 }
 

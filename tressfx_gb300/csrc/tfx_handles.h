@@ -48,6 +48,9 @@ struct tfx_sdf_t {
     int nverts = 0;
     const uint32_t* idx = nullptr;
     int ntri = 0;
+    tfx::TriJob* jobs = nullptr;   // the construct's scratch, for meshes of up to jobsCap triangles
+    int64_t jobsCap = 0;
+    std::vector<void*> jobArrays;  // it and the smaller ones before it
 };
 
 struct tfx_mesh_t {

@@ -55,7 +55,17 @@ cudaError_t launch_local_shape(const HairView& h, cudaStream_t s);
 cudaError_t launch_length_wind(const HairView& h, cudaStream_t s);
 cudaError_t launch_follow(const HairView& h, cudaStream_t s);
 
-cudaError_t launch_sdf_initialize(uint32_t* sdf, int64_t cells, cudaStream_t s);
+struct TriJob;   // tfx_sdf_math.cuh: what the construct keeps of a triangle
+size_t sdf_job_bytes();
+bool sdf_takes_jobs(int64_t tris);   // the construct of a launch over this many triangles reads a job array
+// The words' initial value and, with `jobs`, the job of every triangle.
+cudaError_t launch_sdf_initialize(uint32_t* sdf, int64_t cells, cudaStream_t s, const SdfGrid* g = nullptr,
+                                  const float4* mesh = nullptr, const uint32_t* idx = nullptr, int ntri = 0,
+                                  TriJob* jobs = nullptr);
+cudaError_t launch_sdf_jobs(TriJob* jobs, uint32_t* sdf, const SdfGrid& g, const float4* mesh, const uint32_t* idx, int ntri,
+                            cudaStream_t s);
+// The construct over jobs made beforehand, and the one that needs no job array.
+cudaError_t launch_sdf_construct_jobs(const TriJob* jobs, int ntri, cudaStream_t s);
 cudaError_t launch_sdf_construct(uint32_t* sdf, const SdfGrid& g, const float4* mesh, const uint32_t* idx,
                                  int ntri, cudaStream_t s);
 cudaError_t launch_sdf_finalize(uint32_t* sdf, int64_t cells, cudaStream_t s);

@@ -5,6 +5,7 @@
 // over the encoding = min |d|, ties to the positive value) and plain floats after Finalize.
 // atomicMin is order independent, and the distance arithmetic below is the reference's in the
 // same order with no FMA contraction, so the finished grid matches the oracle bit for bit.
+#include <algorithm>
 #include <atomic>
 
 #include "tfx_sdf_math.cuh"
@@ -12,34 +13,52 @@
 namespace tfx {
 
 // --------------------------------------------------------------------------------------------
-// InitializeSignedDistanceField, :301-312 (vectorised: 4 cells per 16 B store)
-__global__ void __launch_bounds__(256) k_sdf_initialize(uint32_t* __restrict__ sdf, long long cells) {
+__device__ __forceinline__ TriJob plain_job(uint32_t* sdf, const SdfGrid& g, const float4* __restrict__ mesh,
+                                            const uint32_t* __restrict__ idx, int t) {
+    const float3 x0 = xyz(__ldg(mesh + 2 * (size_t)__ldg(idx + 3 * (size_t)t + 0)));
+    const float3 x1 = xyz(__ldg(mesh + 2 * (size_t)__ldg(idx + 3 * (size_t)t + 1)));
+    const float3 x2 = xyz(__ldg(mesh + 2 * (size_t)__ldg(idx + 3 * (size_t)t + 2)));
+    return tri_job(g, sdf, x0, x1, x2);
+}
+
+// InitializeSignedDistanceField, :301-312 (vectorised: 4 cells per 16 B store), with the job of every
+// triangle beside it when there is a job array.
+__global__ void __launch_bounds__(256) k_sdf_initialize(uint32_t* __restrict__ sdf, long long cells, SdfGrid g,
+                                                        const float4* __restrict__ mesh, const uint32_t* __restrict__ idx,
+                                                        int ntri, TriJob* __restrict__ jobs) {
     const uint32_t v = float_flip3(1e10f);
     const long long n4 = cells >> 2;
     const long long stride = (long long)gridDim.x * blockDim.x;
+    const long long me = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    for (long long t = me; t < ntri; t += stride) jobs[t] = plain_job(sdf, g, mesh, idx, (int)t);
     uint4* s4 = reinterpret_cast<uint4*>(sdf);
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += stride) s4[i] = make_uint4(v, v, v, v);
-    for (long long i = (n4 << 2) + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < cells; i += stride) sdf[i] = v;
+    for (long long i = me; i < n4; i += stride) s4[i] = make_uint4(v, v, v, v);
+    for (long long i = (n4 << 2) + me; i < cells; i += stride) sdf[i] = v;
+}
+
+// ConstructSignedDistanceField, :329-397, over the jobs made beforehand.
+__global__ void __launch_bounds__(128, kConstructBlocksPerSM) k_sdf_construct_jobs(const TriJob* __restrict__ jobs, int ntri) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const SdfWarpArea area = sdf_warp_area(smem, warp, kSdfJobsAhead);
+    sdf_construct_jobs_warp(area, jobs, ntri, blockIdx.x * 4 + warp, gridDim.x * 4, lane);
 }
 
 // ConstructSignedDistanceField, :329-397.  Each warp takes chunks of `per` (<= 32) consecutive
-// triangles (sdf_construct_chunk_warp: STAGED, lane k makes the job of the chunk's k-th triangle), then
+// triangles (sdf_construct_chunk_warp: lane k makes the job of the chunk's k-th triangle), then
 // runs the triangles' cell loops in turn; the warps stride over the chunks.
-template <bool STAGED>
 __global__ void __launch_bounds__(128) k_sdf_construct(uint32_t* __restrict__ sdf, SdfGrid g,
                                                        const float4* __restrict__ mesh,
                                                        const uint32_t* __restrict__ idx, int ntri, int per) {
-    __shared__ TriJob jobs[STAGED ? 4 : 1][STAGED ? kTriJobsPerWarp : 1];
+    extern __shared__ __align__(16) unsigned char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    SdfWarpArea area = sdf_warp_area(smem, warp, per);
     const int warpsTotal = gridDim.x * (blockDim.x >> 5);
     const int chunks = (ntri + per - 1) / per;
     for (int k = blockIdx.x * (blockDim.x >> 5) + warp; k < chunks; k += warpsTotal) {
         const int first = k * per;
-        sdf_construct_chunk_warp<STAGED>(jobs[STAGED ? warp : 0], first, min(per, ntri - first), lane, [&](int t) {
-            const float3 x0 = xyz(__ldg(mesh + 2 * (size_t)__ldg(idx + 3 * t + 0)));
-            const float3 x1 = xyz(__ldg(mesh + 2 * (size_t)__ldg(idx + 3 * t + 1)));
-            const float3 x2 = xyz(__ldg(mesh + 2 * (size_t)__ldg(idx + 3 * t + 2)));
-            return tri_job(g, sdf, x0, x1, x2);
+        sdf_construct_chunk_warp(area, first, min(per, ntri - first), lane, [&](int t) {
+            return plain_job(sdf, g, mesh, idx, t);
         });
     }
 }
@@ -159,9 +178,29 @@ static inline unsigned grid_for(long long work, int threads, unsigned cap) {
     return (unsigned)(b > cap ? cap : b);
 }
 
-cudaError_t launch_sdf_initialize(uint32_t* sdf, int64_t cells, cudaStream_t s) {
+size_t sdf_job_bytes() { return sizeof(TriJob); }
+bool sdf_takes_jobs(int64_t tris) { return sdf_wants_jobs(tris, sm_count()); }
+
+cudaError_t launch_sdf_initialize(uint32_t* sdf, int64_t cells, cudaStream_t s, const SdfGrid* g, const float4* mesh,
+                                  const uint32_t* idx, int ntri, TriJob* jobs) {
     if (cells <= 0) return cudaSuccess;
-    k_sdf_initialize<<<grid_for((cells + 3) / 4, 256, sm_count() * 16), 256, 0, s>>>(sdf, cells);
+    const int n = jobs ? ntri : 0;
+    const long long work = std::max<long long>((cells + 3) / 4, n);
+    k_sdf_initialize<<<grid_for(work, 256, sm_count() * 16), 256, 0, s>>>(sdf, cells, g ? *g : SdfGrid{}, mesh, idx, n, jobs);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_sdf_jobs(TriJob* jobs, uint32_t* sdf, const SdfGrid& g, const float4* mesh, const uint32_t* idx, int ntri,
+                            cudaStream_t s) {
+    if (ntri <= 0) return cudaSuccess;
+    k_sdf_initialize<<<grid_for(ntri, 256, sm_count() * 16), 256, 0, s>>>(sdf, 0, g, mesh, idx, ntri, jobs);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_sdf_construct_jobs(const TriJob* jobs, int ntri, cudaStream_t s) {
+    if (ntri <= 0) return cudaSuccess;
+    const unsigned blocks = (unsigned)std::min<long long>(((long long)ntri + 3) / 4, (long long)sm_count() * kConstructBlocksPerSM);
+    k_sdf_construct_jobs<<<blocks, 128, sdf_construct_smem(4, kSdfJobsAhead), s>>>(jobs, ntri);
     return cudaGetLastError();
 }
 
@@ -171,10 +210,7 @@ cudaError_t launch_sdf_construct(uint32_t* sdf, const SdfGrid& g, const float4* 
     const int per = sdf_construct_chunk(ntri, sm_count());
     const long long chunks = ((long long)ntri + per - 1) / per;
     const unsigned blocks = (unsigned)std::min<long long>((chunks + 3) / 4, (long long)sm_count() * 64);
-    if (per >= kTriJobsStagedFrom)
-        k_sdf_construct<true><<<blocks, 128, 0, s>>>(sdf, g, mesh, idx, ntri, per);
-    else
-        k_sdf_construct<false><<<blocks, 128, 0, s>>>(sdf, g, mesh, idx, ntri, per);
+    k_sdf_construct<<<blocks, 128, sdf_construct_smem(4, per), s>>>(sdf, g, mesh, idx, ntri, per);
     return cudaGetLastError();
 }
 
