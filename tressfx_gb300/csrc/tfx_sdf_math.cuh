@@ -3,7 +3,6 @@
 // trilinear lookup of src/Shaders/TressFXSDFCollision.hlsl, evaluated in the reference's order.
 #pragma once
 #include "tfx_device_math.cuh"
-#include "tfx_exact_math.cuh"
 #include "tfx_internal.h"
 
 namespace tfx {
