@@ -6,6 +6,11 @@
 // cols 2i+8..}, {row g+8, cols 2i+8..};  B (16 x 8) regs {rows 2i..2i+1, col g}, {rows 2i+8.., col g};
 // C (16 x 8, f32) {row g, cols 2i, 2i+1}, {row g+8, cols 2i, 2i+1}.  The C fragments of n-tiles 2k and
 // 2k+1 are exactly the A fragment of k-tile k of the next layer, so activations never leave registers.
+#include <algorithm>
+#include <cmath>
+#include <type_traits>
+
+#include "tfx_launch.cuh"
 #include "tfx_neural.cuh"
 #include "tfx_sdf_math.cuh"
 
@@ -41,9 +46,6 @@ __device__ __forceinline__ uint32_t silu2(float a, float b) {
     asm("tanh.approx.bf16x2 %0, %1;" : "=r"(t) : "r"(*reinterpret_cast<uint32_t*>(&h)));
     const __nv_bfloat162 r = __hfma2(h, *reinterpret_cast<__nv_bfloat162*>(&t), h);
     return *reinterpret_cast<const uint32_t*>(&r);
-}
-__device__ __forceinline__ float2 unpack_bf16(uint32_t u) {
-    return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&u));
 }
 __device__ __forceinline__ float silu_grad(float z) {
     const float s = __fdividef(1.0f, 1.0f + __expf(-z));
@@ -103,48 +105,16 @@ __device__ __forceinline__ void init_bias(float (&C)[8][4], const float* b, int 
         C[nt][0] = b0; C[nt][1] = b1; C[nt][2] = b0; C[nt][3] = b1;
     }
 }
-// A fragments of the next layer from C, through SiLU or as they are.
-template <bool SILU>
+// A fragments of the next layer from C, through SiLU.
 __device__ __forceinline__ void c_to_a(const float (&C)[8][4], uint32_t (&A)[4][4]) {
 #pragma unroll
     for (int kt = 0; kt < 4; ++kt) {
-        if constexpr (SILU) {
-            A[kt][0] = silu2(C[2 * kt][0], C[2 * kt][1]);
-            A[kt][1] = silu2(C[2 * kt][2], C[2 * kt][3]);
-            A[kt][2] = silu2(C[2 * kt + 1][0], C[2 * kt + 1][1]);
-            A[kt][3] = silu2(C[2 * kt + 1][2], C[2 * kt + 1][3]);
-        } else {
-            A[kt][0] = pack_bf16(C[2 * kt][0], C[2 * kt][1]);
-            A[kt][1] = pack_bf16(C[2 * kt][2], C[2 * kt][3]);
-            A[kt][2] = pack_bf16(C[2 * kt + 1][0], C[2 * kt + 1][1]);
-            A[kt][3] = pack_bf16(C[2 * kt + 1][2], C[2 * kt + 1][3]);
-        }
+        A[kt][0] = silu2(C[2 * kt][0], C[2 * kt][1]);
+        A[kt][1] = silu2(C[2 * kt][2], C[2 * kt][3]);
+        A[kt][2] = silu2(C[2 * kt + 1][0], C[2 * kt + 1][1]);
+        A[kt][3] = silu2(C[2 * kt + 1][2], C[2 * kt + 1][3]);
     }
 }
-// The activations held in A fragments, back in C-fragment order (for storing them).
-__device__ __forceinline__ void a_to_c(const uint32_t (&A)[4][4], float (&H)[8][4]) {
-#pragma unroll
-    for (int kt = 0; kt < 4; ++kt) {
-        float2 v;
-        v = unpack_bf16(A[kt][0]); H[2 * kt][0] = v.x; H[2 * kt][1] = v.y;
-        v = unpack_bf16(A[kt][1]); H[2 * kt][2] = v.x; H[2 * kt][3] = v.y;
-        v = unpack_bf16(A[kt][2]); H[2 * kt + 1][0] = v.x; H[2 * kt + 1][1] = v.y;
-        v = unpack_bf16(A[kt][3]); H[2 * kt + 1][2] = v.x; H[2 * kt + 1][3] = v.y;
-    }
-}
-// C += A (16 x 64) * W^T for a 64-wide layer whose weights are stored [n][k] with row stride RSH.
-__device__ __forceinline__ void layer64(float (&C)[8][4], const uint32_t (&A)[4][4], const __nv_bfloat16* W, int lane) {
-#pragma unroll
-    for (int kt = 0; kt < 4; ++kt)
-#pragma unroll
-        for (int nt = 0; nt < 8; nt += 2) {
-            uint32_t b[4];
-            load_b2(W, RSH, nt, kt, lane, b);
-            mma16816(C[nt], A[kt][0], A[kt][1], A[kt][2], A[kt][3], b[0], b[1]);
-            mma16816(C[nt + 1], A[kt][0], A[kt][1], A[kt][2], A[kt][3], b[2], b[3]);
-        }
-}
-
 // Features of one point into row s of the tile: the lane pair (2s, 2s+1) splits the work.
 __device__ __forceinline__ void write_features(__nv_bfloat16* F, int s, int half, float ux, float uy, float uz, float p0,
                                                float p1, float p2, bool valid) {
@@ -202,70 +172,6 @@ __device__ __forceinline__ void store_pairs(const float (&C)[8][4], int ntiles, 
     }
 }
 
-// Forward pass of the tile in F (16 points).  y0 / y1 = outputs (cells) of rows g / g+8 (valid in lanes
-// with lane % 4 == 0).  With TRAIN, pre-activations go to zsave (per lane, [4][32]) and activations
-// (pair layout) to hout[1..4].
-template <bool TRAIN>
-__device__ __forceinline__ void mlp_forward(const __nv_bfloat16* sW, const float* sB, const __nv_bfloat16* F, int lane,
-                                            float* zsave, uint32_t* const* hout, float& y0, float& y1) {
-    float C[8][4];
-    init_bias(C, sB, lane);
-#pragma unroll 1
-    for (int kt = 0; kt < KIN / 16; ++kt) {
-        uint32_t a[4];
-        load_a(F, RS1, kt, lane, a);
-#pragma unroll
-        for (int nt = 0; nt < 8; nt += 2) {
-            uint32_t b[4];
-            load_b2(sW + OFF_WT1, RS1, nt, kt, lane, b);
-            mma16816(C[nt], a[0], a[1], a[2], a[3], b[0], b[1]);
-            mma16816(C[nt + 1], a[0], a[1], a[2], a[3], b[2], b[3]);
-        }
-    }
-    const int woff[3] = {OFF_WT2, OFF_WT3, OFF_WT4};
-#pragma unroll 1
-    for (int l = 0; l < 3; ++l) {
-        uint32_t A[4][4];
-        c_to_a<true>(C, A);
-        if constexpr (TRAIN) {
-#pragma unroll
-            for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) zsave[l * 32 + nt * 4 + q] = C[nt][q];
-            float H[8][4];
-            a_to_c(A, H);
-            store_pairs(H, 8, hout[l], HID, lane);
-        }
-        init_bias(C, sB + (l + 1) * HID, lane);
-        layer64(C, A, sW + woff[l], lane);
-    }
-    uint32_t A[4][4];
-    c_to_a<true>(C, A);
-    if constexpr (TRAIN) {
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) zsave[3 * 32 + nt * 4 + q] = C[nt][q];
-        float H[8][4];
-        a_to_c(A, H);
-        store_pairs(H, 8, hout[3], HID, lane);
-    }
-    float C5[4];
-    {
-        const int i = lane & 3;
-        const float b0 = sB[4 * HID + 2 * i], b1 = sB[4 * HID + 2 * i + 1];
-        C5[0] = b0; C5[1] = b1; C5[2] = b0; C5[3] = b1;
-    }
-#pragma unroll
-    for (int kt = 0; kt < 4; ++kt) {
-        uint32_t b0, b1;
-        load_b(sW + OFF_WT5, RSH, 0, kt, lane, b0, b1);
-        mma16816(C5, A[kt][0], A[kt][1], A[kt][2], A[kt][3], b0, b1);
-    }
-    y0 = C5[0];
-    y1 = C5[2];
-}
-
 // Inference forward pass of a 32-point tile (two m-tiles sharing every weight fragment): rows
 // g, g+8 of tile 0 and g, g+8 of tile 1 come back in y[0..3] (valid in lanes with lane % 4 == 0).
 __device__ __forceinline__ void mlp_forward32(const __nv_bfloat16* sW, const float* sB, const __nv_bfloat16* F, int lane,
@@ -292,8 +198,8 @@ __device__ __forceinline__ void mlp_forward32(const __nv_bfloat16* sW, const flo
 #pragma unroll 1
     for (int l = 0; l < 3; ++l) {
         uint32_t A0[4][4], A1[4][4];
-        c_to_a<true>(C[0], A0);
-        c_to_a<true>(C[1], A1);
+        c_to_a(C[0], A0);
+        c_to_a(C[1], A1);
         init_bias(C[0], sB + (l + 1) * HID, lane);
         init_bias(C[1], sB + (l + 1) * HID, lane);
         const __nv_bfloat16* W = sW + woff[l];
@@ -310,8 +216,8 @@ __device__ __forceinline__ void mlp_forward32(const __nv_bfloat16* sW, const flo
             }
     }
     uint32_t A0[4][4], A1[4][4];
-    c_to_a<true>(C[0], A0);
-    c_to_a<true>(C[1], A1);
+    c_to_a(C[0], A0);
+    c_to_a(C[1], A1);
     float C5[2][4];
     {
         const int i = lane & 3;
@@ -342,8 +248,11 @@ static_assert(WBF_FWD * 2 % 16 == 0 && WBF_ALL * 2 % 16 == 0, "weight blocks are
 constexpr int TILE_BYTES = 16 * RS1 * 2;
 constexpr int QUERY_WARPS = 4;
 constexpr size_t QUERY_SMEM = (size_t)WBF_FWD * 2 + NBIAS * 4 + QUERY_WARPS * 2 * TILE_BYTES;
-constexpr int TRAIN_WARPS = 4;
-constexpr size_t TRAIN_SMEM = (size_t)WBF_ALL * 2 + NBIAS * 4 + TRAIN_WARPS * (TILE_BYTES + 4 * 32 * 32 * 4);
+// training: a block carries TRAIN_TILES tiles of 16 samples, four warps to a tile
+constexpr int TRAIN_TILES = 4;
+constexpr int TRAIN_THREADS = TRAIN_TILES * 128;
+constexpr int ACT_BYTES = 16 * RSH * 2;   // a tile's activations or gradients of one layer
+constexpr size_t TRAIN_SMEM = (size_t)WBF_ALL * 2 + NBIAS * 4 + TRAIN_TILES * (TILE_BYTES + 2 * ACT_BYTES + 2 * 16 * 4);
 
 // ------------------------------------------------------------------------------------------ query
 template <bool SAMPLES>
@@ -396,7 +305,59 @@ __global__ void __launch_bounds__(QUERY_WARPS * 32) k_nsdf_query(const __nv_bflo
 // One minibatch: forward with saved activations, loss, backward to every layer's pre-activation
 // gradient.  Activations and gradients go to `acts` in the pair layout for k_nsdf_wgrad:
 //   H0 [B/2][KIN], H1..H4 [B/2][64], dZ1..dZ4 [B/2][64], dZ5 [B/2][8]   (32-bit words).
-__global__ void __launch_bounds__(TRAIN_WARPS * 32) k_nsdf_train(const __nv_bfloat16* __restrict__ wbf,
+//
+// Four warps carry a tile of 16 samples, each a quarter of every layer's 64 columns (two n-tiles of the
+// MMA): a minibatch has only batch / 16 tiles (512 at 8,192 samples), so one warp per tile left four warps
+// on an SM and its time was one warp's chain through the ten layers.  A layer's activations pass between
+// the warps through shared memory (bf16, two buffers by turns), its pre-activations stay in registers for
+// the backward pass.  Bound: that chain and the barrier per layer (8,192 samples, ncu: 23.4 -> 11.9 us).
+__device__ __forceinline__ void copy_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+__device__ __forceinline__ void tile_sync(int tile) { asm volatile("bar.sync %0, 128;" ::"r"(tile + 1) : "memory"); }
+
+// Two n-tiles' words (bf16 pairs of columns c0, c0 + 1; [nt][0] row g, [nt][1] row g + 8) into the tile's
+// shared buffer, and as sample pairs into global memory: words of (row 2p, row 2p + 1), column c.
+__device__ __forceinline__ void store_act(const uint32_t (&w)[2][2], __nv_bfloat16* T, uint32_t* out, int wq, int lane) {
+    const int g = lane >> 2, i = lane & 3;
+    const bool even = (g & 1) == 0;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int c0 = (2 * wq + q) * 8 + 2 * i;
+        if (T) {
+            *reinterpret_cast<uint32_t*>(T + g * RSH + c0) = w[q][0];
+            *reinterpret_cast<uint32_t*>(T + (g + 8) * RSH + c0) = w[q][1];
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const uint32_t mine = w[q][r], other = __shfl_xor_sync(0xffffffffu, mine, 4);
+            out[((g + 8 * r) >> 1) * HID + c0 + (even ? 0 : 1)] =
+                even ? __byte_perm(mine, other, 0x5410) : __byte_perm(other, mine, 0x7632);
+        }
+    }
+}
+
+// C += the tile's 16 x 64 operand in T times the two n-tiles of a 64-wide layer's weights ([n][k], stride RSH).
+__device__ __forceinline__ void layer_quarter(float (&C)[2][4], const __nv_bfloat16* T, const __nv_bfloat16* W, int wq, int lane) {
+#pragma unroll
+    for (int kt = 0; kt < 4; ++kt) {
+        uint32_t a[4], b[4];
+        load_a(T, RSH, kt, lane, a);
+        load_b2(W, RSH, 2 * wq, kt, lane, b);
+        mma16816(C[0], a[0], a[1], a[2], a[3], b[0], b[1]);
+        mma16816(C[1], a[0], a[1], a[2], a[3], b[2], b[3]);
+    }
+}
+__device__ __forceinline__ void bias_quarter(float (&C)[2][4], const float* b, int wq, int lane) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const float2 v = *reinterpret_cast<const float2*>(b + (2 * wq + q) * 8 + 2 * (lane & 3));
+        C[q][0] = v.x; C[q][1] = v.y; C[q][2] = v.x; C[q][3] = v.y;
+    }
+}
+
+__global__ void __launch_bounds__(TRAIN_THREADS, 1) k_nsdf_train(const __nv_bfloat16* __restrict__ wbf,
                                                                  const float* __restrict__ bias, Frame fr,
                                                                  const Sample* __restrict__ pool, long long poolSize,
                                                                  int batch, uint32_t seed, uint32_t* __restrict__ acts,
@@ -404,164 +365,265 @@ __global__ void __launch_bounds__(TRAIN_WARPS * 32) k_nsdf_train(const __nv_bflo
     extern __shared__ uint4 smem_t[];
     __nv_bfloat16* sW = reinterpret_cast<__nv_bfloat16*>(smem_t);
     float* sB = reinterpret_cast<float*>(sW + WBF_ALL);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    __nv_bfloat16* sF = reinterpret_cast<__nv_bfloat16*>(sB + NBIAS) + warp * 16 * RS1;
-    float* sZ = reinterpret_cast<float*>(reinterpret_cast<__nv_bfloat16*>(sB + NBIAS) + TRAIN_WARPS * 16 * RS1) +
-                warp * (4 * 32 * 32) + lane * 128;
-    stage_weights<ALL_U4>(smem_t, wbf, sB, bias);
-    __syncthreads();
-
+    const int tg = threadIdx.x >> 7, wq = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31, tid = threadIdx.x & 127;
+    unsigned char* area = reinterpret_cast<unsigned char*>(sB + NBIAS) + (size_t)tg * (TILE_BYTES + 2 * ACT_BYTES + 2 * 16 * 4);
+    __nv_bfloat16* sF = reinterpret_cast<__nv_bfloat16*>(area);
+    __nv_bfloat16* act[2] = {reinterpret_cast<__nv_bfloat16*>(area + TILE_BYTES), reinterpret_cast<__nv_bfloat16*>(area + TILE_BYTES + ACT_BYTES)};
+    float* sT = reinterpret_cast<float*>(area + TILE_BYTES + 2 * ACT_BYTES);   // targets, then weights
     const long long B2 = batch / 2;
     uint32_t* H0 = acts;
-    uint32_t* Hl[4] = {H0 + B2 * KIN, H0 + B2 * KIN + B2 * HID, H0 + B2 * KIN + 2 * B2 * HID, H0 + B2 * KIN + 3 * B2 * HID};
-    uint32_t* dZ[4] = {Hl[3] + B2 * HID, Hl[3] + 2 * B2 * HID, Hl[3] + 3 * B2 * HID, Hl[3] + 4 * B2 * HID};
-    uint32_t* dZ5 = dZ[3] + B2 * HID;
-
-    const int s = lane >> 1, half = lane & 1, g = lane >> 2, i = lane & 3;
-    const int nw = gridDim.x * TRAIN_WARPS;
-    float lossAcc = 0.f;
-    for (int tile = blockIdx.x * TRAIN_WARPS + warp; tile * 16 < batch; tile += nw) {
-        const int b = tile * 16 + s;
-        const uint32_t h = hash32(seed ^ hash32((uint32_t)b * 2654435761u));
-        const long long idx = (long long)(((unsigned long long)h * (unsigned long long)poolSize) >> 32);
-        const Sample S = pool[idx];
-        write_features(sF, s, half, (S.x - fr.cx) * fr.ihx, (S.y - fr.cy) * fr.ihy, (S.z - fr.cz) * fr.ihz,
-                       S.p0 * fr.poseScale, S.p1 * fr.poseScale, S.p2 * fr.poseScale, true);
-        __syncwarp();
-        // H0 in the pair layout
-        uint32_t* h0 = H0 + (long long)tile * 8 * KIN;
-        for (int w = lane; w < 8 * KIN; w += 32) {
-            const int p = w / KIN, f = w - p * KIN;
-            const __nv_bfloat16 lo = sF[(2 * p) * RS1 + f], hi = sF[(2 * p + 1) * RS1 + f];
-            __nv_bfloat162 v; v.x = lo; v.y = hi;
-            h0[w] = *reinterpret_cast<uint32_t*>(&v);
+    uint32_t* H1 = H0 + B2 * KIN;          // H1..H4, then dZ1..dZ4, then dZ5
+    uint32_t* dZ1 = H1 + 4 * B2 * HID;
+    uint32_t* dZ5 = dZ1 + 4 * B2 * HID;
+    const int g = lane >> 2, i = lane & 3;
+    const int s = tid >> 3, part = tid & 7;   // the thread's sample and its eighth of the features
+    auto features = [&](int tile) {   // as write_features, a sample's 18 recurrences over eight threads
+        const uint32_t h = hash32(seed ^ hash32((uint32_t)(tile * 16 + s) * 2654435761u));
+        const Sample S = pool[(long long)(((unsigned long long)h * (unsigned long long)poolSize) >> 32)];
+        const float u[3] = {(S.x - fr.cx) * fr.ihx, (S.y - fr.cy) * fr.ihy, (S.z - fr.cz) * fr.ihz};
+        __nv_bfloat16* row = sF + s * RS1;
+        if (part == 0) {
+            const float f[6] = {u[0], u[1], u[2], S.p0 * fr.poseScale, S.p1 * fr.poseScale, S.p2 * fr.poseScale};
+#pragma unroll
+            for (int k = 0; k < 6; ++k) row[k] = __float2bfloat16(f[k]);
+            sT[s] = S.target;
+            sT[16 + s] = S.weight;
+        } else if (part == 1) {
+#pragma unroll
+            for (int f = NFEAT; f < KIN; ++f) row[f] = __float2bfloat16(0.f);
         }
-        uint32_t* hout[4] = {Hl[0] + (long long)tile * 8 * HID, Hl[1] + (long long)tile * 8 * HID,
-                             Hl[2] + (long long)tile * 8 * HID, Hl[3] + (long long)tile * 8 * HID};
-        float y0, y1;
-        mlp_forward<true>(sW, sB, sF, lane, sZ, hout, y0, y1);
-        __syncwarp();
-        // targets and weights of rows g, g+8 live in lanes 2g(+1), 2(g+8)
-        const float t0 = __shfl_sync(0xffffffffu, S.target, 2 * g), t1 = __shfl_sync(0xffffffffu, S.target, 2 * (g + 8));
-        const float w0 = __shfl_sync(0xffffffffu, S.weight, 2 * g), w1 = __shfl_sync(0xffffffffu, S.weight, 2 * (g + 8));
-        y0 = __shfl_sync(0xffffffffu, y0, lane & ~3);
-        y1 = __shfl_sync(0xffffffffu, y1, lane & ~3);
-        const float e0 = y0 - t0, e1 = y1 - t1;
-        if (i == 0) lossAcc += w0 * e0 * e0 + w1 * e1 * e1;
+        for (int c = part; c < 18; c += 8) {
+            const int k0 = c >= 9 ? NFREQ / 2 : 0, b = (c % 9) / 3, d = c % 3;
+            float sn, cs;
+            sincospi_fast(c_freq[k0 + b] * (d == 0 ? u[0] : d == 1 ? u[1] : u[2]), &sn, &cs);
+            for (int k = k0 + b; k < k0 + NFREQ / 2; k += 3) {
+                *reinterpret_cast<__nv_bfloat162*>(row + 6 + 6 * k + 2 * d) = __floats2bfloat162_rn(sn, cs);
+                const float s2 = 2.0f * sn * cs, c2 = 1.0f - 2.0f * sn * sn;
+                sn = s2; cs = c2;
+            }
+        }
+    };
+    float lossAcc = 0.f;
+    int tile = blockIdx.x * TRAIN_TILES + tg;
+    // the first tile's features need only the samples, which the launch before this one does not write
+    if (tile * 16 < batch) features(tile);
+    after_previous();
+    let_next_in();
+    for (int k = threadIdx.x; k < ALL_U4; k += TRAIN_THREADS) copy_async16(smem_t + k, reinterpret_cast<const uint4*>(wbf) + k);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int k = threadIdx.x; k < NBIAS; k += TRAIN_THREADS) sB[k] = bias[k];
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    for (bool first = true; tile * 16 < batch; tile += gridDim.x * TRAIN_TILES, first = false) {
+        if (!first) {
+            features(tile);
+            tile_sync(tg);
+        }
+        {   // H0 in the pair layout
+            uint32_t* h0 = H0 + (long long)tile * 8 * KIN;
+            for (int w = tid; w < 8 * KIN; w += 128) {
+                const int p = w / KIN, f = w - p * KIN;
+                __nv_bfloat162 v;
+                v.x = sF[(2 * p) * RS1 + f];
+                v.y = sF[(2 * p + 1) * RS1 + f];
+                h0[w] = *reinterpret_cast<uint32_t*>(&v);
+            }
+        }
+        float C[2][4], z[4][8];
+        uint32_t w[2][2];
+        bias_quarter(C, sB, wq, lane);
+#pragma unroll
+        for (int kt = 0; kt < KIN / 16; ++kt) {
+            uint32_t a[4], b[4];
+            load_a(sF, RS1, kt, lane, a);
+            load_b2(sW + OFF_WT1, RS1, 2 * wq, kt, lane, b);
+            mma16816(C[0], a[0], a[1], a[2], a[3], b[0], b[1]);
+            mma16816(C[1], a[0], a[1], a[2], a[3], b[2], b[3]);
+        }
+        const int wt[3] = {OFF_WT2, OFF_WT3, OFF_WT4}, wn[3] = {OFF_WN2, OFF_WN3, OFF_WN4};
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {   // C = pre-activations of layer l + 1
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) z[l][4 * q + e] = C[q][e];
+                w[q][0] = silu2(C[q][0], C[q][1]);
+                w[q][1] = silu2(C[q][2], C[q][3]);
+            }
+            store_act(w, act[l & 1], H1 + l * B2 * HID + (long long)tile * 8 * HID, wq, lane);
+            tile_sync(tg);
+            if (l < 3) {
+                bias_quarter(C, sB + (l + 1) * HID, wq, lane);
+                layer_quarter(C, act[l & 1], sW + wt[l], wq, lane);
+            }
+        }
+        // the output, by every warp: rows g and g + 8 in the lanes with i = 0
+        float C5[4];
+        {
+            const float2 v = *reinterpret_cast<const float2*>(sB + 4 * HID + 2 * i);
+            C5[0] = v.x; C5[1] = v.y; C5[2] = v.x; C5[3] = v.y;
+        }
+#pragma unroll
+        for (int kt = 0; kt < 4; ++kt) {
+            uint32_t a[4], b0, b1;
+            load_a(act[1], RSH, kt, lane, a);
+            load_b(sW + OFF_WT5, RSH, 0, kt, lane, b0, b1);
+            mma16816(C5, a[0], a[1], a[2], a[3], b0, b1);
+        }
+        const float y0 = __shfl_sync(0xffffffffu, C5[0], lane & ~3), y1 = __shfl_sync(0xffffffffu, C5[2], lane & ~3);
+        const float e0 = y0 - sT[g], e1 = y1 - sT[g + 8], w0 = sT[16 + g], w1 = sT[16 + g + 8];
         const float inv = 1.0f / (float)batch;
         const float dy0 = 2.0f * w0 * e0 * inv, dy1 = 2.0f * w1 * e1 * inv;
-        float D[8][4];
-        // dZ5 (column 0 only)
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) D[nt][q] = 0.f;
-        if (i == 0) { D[0][0] = dy0; D[0][2] = dy1; }
-        store_pairs(D, 1, dZ5 + (long long)tile * 8 * OUTN, OUTN, lane);
+        if (wq == 0) {
+            if (i == 0) lossAcc += w0 * e0 * e0 + w1 * e1 * e1;
+            float D5[8][4] = {};
+            if (i == 0) { D5[0][0] = dy0; D5[0][2] = dy1; }   // column 0 only
+            store_pairs(D5, 1, dZ5 + (long long)tile * 8 * OUTN, OUTN, lane);
+        }
         // dH4 = dy * W5[:, 0], then through SiLU
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-            const int n0 = nt * 8 + 2 * i;
+        for (int q = 0; q < 2; ++q) {
+            const int n0 = (2 * wq + q) * 8 + 2 * i;
             const float w50 = __bfloat162float(sW[OFF_WT5 + n0]), w51 = __bfloat162float(sW[OFF_WT5 + n0 + 1]);
-            D[nt][0] = dy0 * w50 * silu_grad(sZ[3 * 32 + nt * 4 + 0]);
-            D[nt][1] = dy0 * w51 * silu_grad(sZ[3 * 32 + nt * 4 + 1]);
-            D[nt][2] = dy1 * w50 * silu_grad(sZ[3 * 32 + nt * 4 + 2]);
-            D[nt][3] = dy1 * w51 * silu_grad(sZ[3 * 32 + nt * 4 + 3]);
+            C[q][0] = dy0 * w50 * silu_grad(z[3][4 * q + 0]);
+            C[q][1] = dy0 * w51 * silu_grad(z[3][4 * q + 1]);
+            C[q][2] = dy1 * w50 * silu_grad(z[3][4 * q + 2]);
+            C[q][3] = dy1 * w51 * silu_grad(z[3][4 * q + 3]);
         }
-        const int wn[3] = {OFF_WN4, OFF_WN3, OFF_WN2};
-#pragma unroll 1
-        for (int l = 3; l >= 1; --l) {   // D = dZ of layer l+1 (1-based); produce dZ of layer l
-            store_pairs(D, 8, dZ[l] + (long long)tile * 8 * HID, HID, lane);
-            uint32_t A[4][4];
-            c_to_a<false>(D, A);
 #pragma unroll
-            for (int nt = 0; nt < 8; ++nt)
+        for (int l = 3; l >= 0; --l) {   // C = dZ of layer l + 1; produce dZ of layer l
 #pragma unroll
-                for (int q = 0; q < 4; ++q) D[nt][q] = 0.f;
-            layer64(D, A, sW + wn[3 - l], lane);
+            for (int q = 0; q < 2; ++q) {
+                w[q][0] = pack_bf16(C[q][0], C[q][1]);
+                w[q][1] = pack_bf16(C[q][2], C[q][3]);
+            }
+            // act[1] was last read for the output, act[0] before the barrier of layer 4
+            __nv_bfloat16* T = act[(l & 1) ^ 1];
+            store_act(w, l > 0 ? T : nullptr, dZ1 + l * B2 * HID + (long long)tile * 8 * HID, wq, lane);
+            if (l == 0) break;
+            tile_sync(tg);
 #pragma unroll
-            for (int nt = 0; nt < 8; ++nt)
+            for (int q = 0; q < 2; ++q)
 #pragma unroll
-                for (int q = 0; q < 4; ++q) D[nt][q] *= silu_grad(sZ[(l - 1) * 32 + nt * 4 + q]);
+                for (int e = 0; e < 4; ++e) C[q][e] = 0.f;
+            layer_quarter(C, T, sW + wn[l - 1], wq, lane);
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) C[q][e] *= silu_grad(z[l - 1][4 * q + e]);
         }
-        store_pairs(D, 8, dZ[0] + (long long)tile * 8 * HID, HID, lane);
-        __syncwarp();
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) lossAcc += __shfl_xor_sync(0xffffffffu, lossAcc, o);
-    if (lane == 0) atomicAdd(lossSum, lossAcc);
+    if (wq == 0 && lane == 0) atomicAdd(lossSum, lossAcc);
 }
 
-// Weight and bias gradients, all five layers in one launch: dW_l = H_{l-1}^T dZ_l, db_l = 1^T dZ_l,
-// summed over the batch.  A warp owns one 16-row tile of one layer (the last tile of a layer is the
-// bias row) for one chunk of samples, and adds its sums into `grads` (parameter layout).
-constexpr int WG_CHUNK = 512;
-__global__ void __launch_bounds__(128) k_nsdf_wgrad(const uint32_t* __restrict__ acts, int batch, float* __restrict__ grads) {
-    const int warpGlobal = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    const int chunks = batch / WG_CHUNK;
-    // jobs: layer 1 has 7 + 1 row tiles, layers 2..5 have 4 + 1
-    const int tilesPerChunk = 8 + 4 * 5;
-    if (warpGlobal >= tilesPerChunk * chunks) return;
-    const int chunk = warpGlobal / tilesPerChunk;
-    int job = warpGlobal - chunk * tilesPerChunk;
-    int layer, mt;
-    if (job < 8) { layer = 1; mt = job; } else { job -= 8; layer = 2 + job / 5; mt = job % 5; }
+// Weight and bias gradients, all five layers in one launch: dW_l = H_{l-1}^T dZ_l, db_l = 1^T dZ_l.  A
+// block owns one layer for a part of the batch (`rounds` times 128 samples): it brings both operands into
+// shared memory whole (16-byte copies; rows padded by eight words, which keeps the fragment reads free of
+// bank conflicts), its warps multiply 16-row tiles -- layer 1 has seven of 64 columns, layers 2 to 4 four
+// of which two warps take 32 columns each, layer 5 four of eight -- and it writes its sums to the part's
+// own copy of the gradient, which k_nsdf_adam adds up: the sums do not depend on the order of the blocks.
+// Bound: the latency of the copies.  8,192 samples (ncu): one warp per 16-row tile and 512 samples, added
+// with atomics, 42 us; this split with vector atomics from 64 blocks a word 18 us; as it is 10 us.  32 or 16
+// parts in place of 64 made the whole step slower (21.6 and 26.3 against 20.1 us).
+constexpr int WG_SAMPLES = 128;
+constexpr int WG_PAIRS = WG_SAMPLES / 2;
+constexpr int WG_THREADS = 256;
+constexpr int WG_PAD = 8;
+constexpr size_t WG_SMEM = sizeof(uint32_t) * WG_PAIRS * (KIN + WG_PAD + HID + WG_PAD);
+constexpr int WG_CHUNK = 512;   // batches are a multiple of this
+
+__global__ void __launch_bounds__(WG_THREADS) k_nsdf_wgrad(const uint32_t* __restrict__ acts, int batch, int rounds,
+                                                           float* __restrict__ parts) {
+    extern __shared__ uint4 smem_w[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int layer = blockIdx.x % 5 + 1, part = blockIdx.x / 5;
+    const int chunks = batch / WG_SAMPLES, chunk0 = part * rounds, chunk1 = min(chunk0 + rounds, chunks);
+    float* grads = parts + (size_t)part * NPARAM;
     const long long B2 = batch / 2;
-    const uint32_t* H0 = acts;
-    const uint32_t* Hprev;
-    const uint32_t* dZ;
-    int Fin, Fout, pW, pB;
-    const uint32_t* Hl1 = H0 + B2 * KIN;
-    const uint32_t* dZ1 = Hl1 + 4 * B2 * HID;
-    switch (layer) {
-        case 1: Hprev = H0; Fin = KIN; dZ = dZ1; Fout = HID; pW = P_W1; pB = P_B1; break;
-        case 2: Hprev = Hl1; Fin = HID; dZ = dZ1 + B2 * HID; Fout = HID; pW = P_W2; pB = P_B2; break;
-        case 3: Hprev = Hl1 + B2 * HID; Fin = HID; dZ = dZ1 + 2 * B2 * HID; Fout = HID; pW = P_W3; pB = P_B3; break;
-        case 4: Hprev = Hl1 + 2 * B2 * HID; Fin = HID; dZ = dZ1 + 3 * B2 * HID; Fout = HID; pW = P_W4; pB = P_B4; break;
-        default: Hprev = Hl1 + 3 * B2 * HID; Fin = HID; dZ = dZ1 + 4 * B2 * HID; Fout = OUTN; pW = P_W5; pB = P_B5; break;
-    }
-    const bool biasTile = mt == Fin / 16;
-    const int ntiles = Fout / 8;
+    const uint32_t* H1 = acts + B2 * KIN;
+    const uint32_t* dZ1 = H1 + 4 * B2 * HID;
+    const int fin = layer == 1 ? KIN : HID, fout = layer == 5 ? OUTN : HID;
+    const uint32_t* Hp = layer == 1 ? acts : H1 + (layer - 2) * B2 * HID;
+    const uint32_t* dZ = dZ1 + (layer - 1) * B2 * HID;
+    const int pW = layer == 1 ? P_W1 : layer == 2 ? P_W2 : layer == 3 ? P_W3 : layer == 4 ? P_W4 : P_W5;
+    const int pB = layer == 1 ? P_B1 : layer == 2 ? P_B2 : layer == 3 ? P_B3 : layer == 4 ? P_B4 : P_B5;
+    const int sa = fin + WG_PAD, sb = fout + WG_PAD;
+    uint32_t* A = reinterpret_cast<uint32_t*>(smem_w);
+    uint32_t* B = A + WG_PAIRS * sa;
     const int g = lane >> 2, i = lane & 3;
-    float C[8][4];
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) C[nt][q] = 0.f;
-    const uint32_t one2 = pack_bf16(1.0f, 1.0f);
-    for (int k0 = chunk * WG_CHUNK; k0 < (chunk + 1) * WG_CHUNK; k0 += 16) {
-        const long long p0 = k0 / 2 + i, p1 = p0 + 4;   // sample pairs of k rows 2i.. and 2i+8..
-        uint32_t a0, a1, a2, a3;
-        if (biasTile) {
-            a0 = g == 0 ? one2 : 0u; a1 = 0u; a2 = g == 0 ? one2 : 0u; a3 = 0u;
-        } else {
-            const int f = mt * 16 + g;
-            a0 = Hprev[p0 * Fin + f];
-            a1 = Hprev[p0 * Fin + f + 8];
-            a2 = Hprev[p1 * Fin + f];
-            a3 = Hprev[p1 * Fin + f + 8];
+    after_previous();
+    let_next_in();
+    auto bring = [&](int chunk) {
+        const uint32_t* a = Hp + (long long)chunk * WG_PAIRS * fin;
+        const uint32_t* b = dZ + (long long)chunk * WG_PAIRS * fout;
+        for (int k = threadIdx.x; k < WG_PAIRS * fin / 4; k += WG_THREADS) {
+            const int r = k / (fin / 4), c = 4 * (k - r * (fin / 4));
+            copy_async16(A + r * sa + c, a + r * fin + c);
         }
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-            if (nt >= ntiles) break;
-            const uint32_t b0 = dZ[p0 * Fout + nt * 8 + g], b1 = dZ[p1 * Fout + nt * 8 + g];
-            mma16816(C[nt], a0, a1, a2, a3, b0, b1);
+        for (int k = threadIdx.x; k < WG_PAIRS * fout / 4; k += WG_THREADS) {
+            const int r = k / (fout / 4), c = 4 * (k - r * (fout / 4));
+            copy_async16(B + r * sb + c, b + r * fout + c);
         }
-    }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+    };
+    // every warp of the block goes through the same rounds; `rows`: it has a tile (mt, columns n0..)
+    auto tile = [&](bool rows, int mt, int n0, auto ntiles) {
+        constexpr int NT = decltype(ntiles)::value;
+        constexpr int BC = 8;   // bias columns of a warp (all 64 of layer 1 over eight warps as well)
+        float C[NT][4], bias[BC];
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-        if (nt >= ntiles) break;
-        const int n0 = nt * 8 + 2 * i;
-        if (biasTile) {
-            if (g == 0) { atomicAdd(grads + pB + n0, C[nt][0]); atomicAdd(grads + pB + n0 + 1, C[nt][1]); }
-        } else {
-            const int m0 = mt * 16 + g;
-            atomicAdd(grads + pW + m0 * Fout + n0, C[nt][0]);
-            atomicAdd(grads + pW + m0 * Fout + n0 + 1, C[nt][1]);
-            atomicAdd(grads + pW + (m0 + 8) * Fout + n0, C[nt][2]);
-            atomicAdd(grads + pW + (m0 + 8) * Fout + n0 + 1, C[nt][3]);
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) C[nt][q] = 0.f;
+#pragma unroll
+        for (int c = 0; c < BC; ++c) bias[c] = 0.f;
+        const int bc0 = warp * BC;
+        for (int chunk = chunk0; chunk < chunk1; ++chunk) {
+            if (chunk > chunk0) __syncthreads();   // the last round's reads come before its copies
+            bring(chunk);
+            if (rows) {
+#pragma unroll
+                for (int ks = 0; ks < WG_SAMPLES / 16; ++ks) {
+                    const uint32_t* a = A + (8 * ks + i) * sa + mt * 16 + g;   // sample pairs of k rows 2i.. and 2i+8..
+                    const uint32_t* b = B + (8 * ks + i) * sb + n0 + g;
+#pragma unroll
+                    for (int nt = 0; nt < NT; ++nt)
+                        mma16816(C[nt], a[0], a[8], a[4 * sa], a[4 * sa + 8], b[nt * 8], b[4 * sb + nt * 8]);
+                }
+            }
+            if (bc0 < fout)
+#pragma unroll
+                for (int p = 0; p < WG_PAIRS; p += 32) {
+                    const uint4* b = reinterpret_cast<const uint4*>(B + (p + lane) * sb + bc0);
+                    const uint4 v[2] = {b[0], b[1]};
+                    const uint32_t* u = reinterpret_cast<const uint32_t*>(v);
+#pragma unroll
+                    for (int c = 0; c < BC; ++c) bias[c] += __uint_as_float(u[c] << 16) + __uint_as_float(u[c] & 0xffff0000u);
+                }
         }
-    }
+        if (rows) {
+            float* out = grads + pW + (mt * 16 + g) * fout + n0 + 2 * i;
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+                *reinterpret_cast<float2*>(out + nt * 8) = make_float2(C[nt][0], C[nt][1]);
+                *reinterpret_cast<float2*>(out + 8 * fout + nt * 8) = make_float2(C[nt][2], C[nt][3]);
+            }
+        }
+        if (bc0 < fout)
+#pragma unroll
+            for (int c = 0; c < BC; ++c) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) bias[c] += __shfl_xor_sync(0xffffffffu, bias[c], o);
+                if (lane == 0) grads[pB + bc0 + c] = bias[c];
+            }
+    };
+    if (layer == 1) tile(warp < KIN / 16, warp, 0, std::integral_constant<int, 8>{});
+    else if (layer < 5) tile(true, warp >> 1, (warp & 1) * 32, std::integral_constant<int, 4>{});
+    else tile(warp < 4, warp, 0, std::integral_constant<int, 1>{});
 }
 
 // Parameter p's places in the bf16 weight block / bias vector.
@@ -592,27 +654,56 @@ __device__ __forceinline__ void publish(int p, float w, __nv_bfloat16* wbf, floa
     }
 }
 
-// Adam (Kingma & Ba 2015) on the fp32 master parameters, then the bf16 / bias copies the kernels read.
-__global__ void k_nsdf_adam(float* __restrict__ params, const float* __restrict__ grads, float* __restrict__ m,
-                            float* __restrict__ v, int step, float lr, float gradScale, __nv_bfloat16* __restrict__ wbf,
-                            float* __restrict__ bias) {
+// The bf16 / bias copies of the fp32 master parameters, which the kernels read.
+__global__ void k_nsdf_publish(const float* __restrict__ params, __nv_bfloat16* __restrict__ wbf, float* __restrict__ bias) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= NPARAM) return;
-    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    float w = params[p];
-    if (step > 0) {
-        const float gr = grads[p] * gradScale;
-        const float mm = b1 * m[p] + (1.0f - b1) * gr;
-        const float vv = b2 * v[p] + (1.0f - b2) * gr * gr;
-        m[p] = mm; v[p] = vv;
-        const float mh = mm / (1.0f - powf(b1, (float)step)), vh = vv / (1.0f - powf(b2, (float)step));
-        w -= lr * mh / (sqrtf(vh) + eps);
-        // the padding rows of the first layer and the unused output columns stay zero
-        const bool pad = (p < P_B1 && p / HID >= NFEAT) || (p >= P_W5 && p < P_B5 && (p - P_W5) % OUTN != 0) ||
-                         (p >= P_B5 && p != P_B5);
-        if (pad) w = 0.f;
-        params[p] = w;
+    if (p < NPARAM) publish(p, params[p], wbf, bias);
+}
+
+// The gradient as the sum of its `nparts` parts, Adam (Kingma & Ba 2015) on the fp32 master parameters, then
+// their copies.  Eight lanes share four consecutive parameters: each adds an eighth of the parts, the first
+// four update one parameter each.  corr1, corr2: 1 - b1^step and 1 - b2^step.
+constexpr int ADAM_THREADS = 256;
+static_assert(NPARAM % 4 == 0, "parameters are summed four at a time");
+__global__ void __launch_bounds__(ADAM_THREADS) k_nsdf_adam(float* __restrict__ params, const float* __restrict__ parts, int nparts,
+                                                            float* __restrict__ grads, float* __restrict__ m, float* __restrict__ v,
+                                                            float corr1, float corr2, float lr, __nv_bfloat16* __restrict__ wbf,
+                                                            float* __restrict__ bias) {
+    const int t = blockIdx.x * ADAM_THREADS + threadIdx.x;
+    const int quad = t >> 3, lane8 = t & 7;
+    const bool mine = quad < NPARAM / 4, update = mine && lane8 < 4;
+    const int p = 4 * quad + lane8;
+    // written by the step before, which ended before the launches this one follows began
+    const float m0 = update ? m[p] : 0.f, v0 = update ? v[p] : 0.f, w0 = update ? params[p] : 0.f;
+    after_previous();
+    let_next_in();
+    float4 gr = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (mine) {
+        const float4* src = reinterpret_cast<const float4*>(parts) + quad;
+#pragma unroll 8
+        for (int c = lane8; c < nparts; c += 8) {
+            const float4 x = src[(size_t)c * (NPARAM / 4)];
+            gr.x += x.x; gr.y += x.y; gr.z += x.z; gr.w += x.w;
+        }
     }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+        gr.x += __shfl_xor_sync(0xffffffffu, gr.x, o); gr.y += __shfl_xor_sync(0xffffffffu, gr.y, o);
+        gr.z += __shfl_xor_sync(0xffffffffu, gr.z, o); gr.w += __shfl_xor_sync(0xffffffffu, gr.w, o);
+    }
+    if (!update) return;
+    const float g = lane8 == 0 ? gr.x : lane8 == 1 ? gr.y : lane8 == 2 ? gr.z : gr.w;
+    grads[p] = g;
+    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+    const float mm = b1 * m0 + (1.0f - b1) * g;
+    const float vv = b2 * v0 + (1.0f - b2) * g * g;
+    m[p] = mm; v[p] = vv;
+    const float mh = mm / corr1, vh = vv / corr2;
+    float w = w0 - lr * mh / (sqrtf(vh) + eps);
+    // the padding rows of the first layer and the unused output columns stay zero
+    const bool pad = (p < P_B1 && p / HID >= NFEAT) || (p >= P_W5 && p < P_B5 && (p - P_W5) % OUTN != 0) || (p >= P_B5 && p != P_B5);
+    if (pad) w = 0.f;
+    params[p] = w;
     publish(p, w, wbf, bias);
 }
 
@@ -668,7 +759,11 @@ __global__ void k_nsdf_sample(const float4* __restrict__ mesh, int nverts, const
 
 }  // namespace
 
-size_t acts_elements(int batch) { return (size_t)batch * (KIN + 8 * HID + OUTN); }
+// A training step's scratch: the minibatch's activations and gradients in the pair layout, then the parts
+// of the weight gradient (at most TRAIN_PARTS, one per 128 samples or more).
+constexpr int TRAIN_PARTS = 64;
+static size_t acts_words(int batch) { return (size_t)batch / 2 * (KIN + 8 * HID + OUTN); }
+size_t train_scratch_bytes(int batch) { return 4 * acts_words(batch) + sizeof(float) * (size_t)NPARAM * TRAIN_PARTS; }
 
 cudaError_t launch_query(const __nv_bfloat16* wbf, const float* bias, const Frame& fr, const float4* points, int count,
                          Pose pose, float* out, cudaStream_t s) {
@@ -693,26 +788,33 @@ cudaError_t launch_query_samples(const __nv_bfloat16* wbf, const float* bias, co
     return cudaGetLastError();
 }
 
-cudaError_t launch_train_step(const __nv_bfloat16* wbf, const float* bias, const Frame& fr, const Sample* pool,
-                              long long poolSize, int batch, uint32_t seed, __nv_bfloat16* acts, float* grads,
-                              float* lossSum, cudaStream_t s) {
-    if (batch <= 0 || batch % WG_CHUNK != 0 || poolSize <= 0) return cudaErrorInvalidValue;
+cudaError_t launch_train_step(const TrainStep& t, cudaStream_t s) {
+    if (t.batch <= 0 || t.batch % WG_CHUNK != 0 || t.poolSize <= 0) return cudaErrorInvalidValue;
     cudaError_t e = cudaFuncSetAttribute(k_nsdf_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TRAIN_SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_nsdf_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WG_SMEM);
     if (e != cudaSuccess) return e;
-    const int tiles = batch / 16;
-    const int blocks = std::min((tiles + TRAIN_WARPS - 1) / TRAIN_WARPS, sm_count() * 2);
-    k_nsdf_train<<<blocks, TRAIN_WARPS * 32, TRAIN_SMEM, s>>>(wbf, bias, fr, pool, poolSize, batch, seed,
-                                                             reinterpret_cast<uint32_t*>(acts), lossSum);
-    e = cudaMemsetAsync(grads, 0, sizeof(float) * NPARAM, s);
+    uint32_t* acts = static_cast<uint32_t*>(t.scratch);
+    float* parts = reinterpret_cast<float*>(acts + acts_words(t.batch));
+    const int blocks = std::min(t.batch / (16 * TRAIN_TILES), sm_count());
+    if (t.first) {
+        k_nsdf_train<<<blocks, TRAIN_THREADS, TRAIN_SMEM, s>>>(t.wbf, t.bias, t.fr, t.pool, t.poolSize, t.batch, t.seed, acts, t.lossSum);
+        e = cudaGetLastError();
+    } else {
+        e = launch_after(k_nsdf_train, blocks, TRAIN_THREADS, TRAIN_SMEM, s, t.wbf, t.bias, t.fr, t.pool, t.poolSize, t.batch,
+                         t.seed, acts, t.lossSum);
+    }
     if (e != cudaSuccess) return e;
-    const int warps = (batch / WG_CHUNK) * (8 + 4 * 5);
-    k_nsdf_wgrad<<<(warps + 3) / 4, 128, 0, s>>>(reinterpret_cast<const uint32_t*>(acts), batch, grads);
-    return cudaGetLastError();
+    const int chunks = t.batch / WG_SAMPLES, rounds = (chunks + TRAIN_PARTS - 1) / TRAIN_PARTS, nparts = (chunks + rounds - 1) / rounds;
+    e = launch_after(k_nsdf_wgrad, (unsigned)nparts * 5, WG_THREADS, WG_SMEM, s, acts, t.batch, rounds, parts);
+    if (e != cudaSuccess) return e;
+    const float corr1 = (float)(1.0 - std::pow((double)0.9f, (double)t.step));
+    const float corr2 = (float)(1.0 - std::pow((double)0.999f, (double)t.step));
+    return launch_after(k_nsdf_adam, (NPARAM / 4 * 8 + ADAM_THREADS - 1) / ADAM_THREADS, ADAM_THREADS, 0, s, t.params, parts, nparts,
+                        t.grads, t.m, t.v, corr1, corr2, t.lr, t.wbf, t.bias);
 }
 
-cudaError_t launch_adam(float* params, const float* grads, float* m, float* v, int step, float lr, float gradScale,
-                        __nv_bfloat16* wbf, float* bias, cudaStream_t s) {
-    k_nsdf_adam<<<(NPARAM + 255) / 256, 256, 0, s>>>(params, grads, m, v, step, lr, gradScale, wbf, bias);
+cudaError_t launch_publish(const float* params, __nv_bfloat16* wbf, float* bias, cudaStream_t s) {
+    k_nsdf_publish<<<(NPARAM + 255) / 256, 256, 0, s>>>(params, wbf, bias);
     return cudaGetLastError();
 }
 
@@ -720,8 +822,7 @@ cudaError_t launch_init_params(float* params, uint32_t seed, __nv_bfloat16* wbf,
     cudaError_t e = cudaMemsetAsync(wbf, 0, sizeof(__nv_bfloat16) * WBF_ALL, s);
     if (e != cudaSuccess) return e;
     k_nsdf_init<<<(NPARAM + 255) / 256, 256, 0, s>>>(params, seed);
-    k_nsdf_adam<<<(NPARAM + 255) / 256, 256, 0, s>>>(params, nullptr, nullptr, nullptr, 0, 0.f, 0.f, wbf, bias);
-    return cudaGetLastError();
+    return launch_publish(params, wbf, bias, s);
 }
 
 cudaError_t launch_sample(const float4* mesh, int nverts, const float* grid, const SdfGrid& g, float band, float sigma,

@@ -68,11 +68,26 @@ cudaError_t launch_query(const __nv_bfloat16* wbf, const float* bias, const Fram
                          Pose pose, float* out, cudaStream_t s);
 cudaError_t launch_query_samples(const __nv_bfloat16* wbf, const float* bias, const Frame& fr, const Sample* samples,
                                  int count, float* out, cudaStream_t s);
-cudaError_t launch_train_step(const __nv_bfloat16* wbf, const float* bias, const Frame& fr, const Sample* pool,
-                              long long poolSize, int batch, uint32_t seed, __nv_bfloat16* acts, float* grads,
-                              float* lossSum, cudaStream_t s);
-cudaError_t launch_adam(float* params, const float* grads, float* m, float* v, int step, float lr, float gradScale,
-                        __nv_bfloat16* wbf, float* bias, cudaStream_t s);
+// One Adam step on a minibatch drawn from the pool (`batch` a multiple of 512): forward and backward, weight
+// gradients, update.  `scratch`: train_scratch_bytes(batch), 16-byte aligned.
+struct TrainStep {
+    __nv_bfloat16* wbf;
+    float* bias;
+    Frame fr;
+    const Sample* pool;
+    long long poolSize;
+    int batch;
+    uint32_t seed;
+    void* scratch;
+    float *params, *grads, *m, *v, *lossSum;
+    int step;        // from 1
+    float lr;
+    bool first;      // the launch before this step on the stream is not a step's (it may have written the samples)
+};
+cudaError_t launch_train_step(const TrainStep& t, cudaStream_t s);
+size_t train_scratch_bytes(int batch);
+// The copies of the master parameters that the kernels read.
+cudaError_t launch_publish(const float* params, __nv_bfloat16* wbf, float* bias, cudaStream_t s);
 cudaError_t launch_init_params(float* params, uint32_t seed, __nv_bfloat16* wbf, float* bias, cudaStream_t s);
 // `count` training samples for one pose: near the skinned mesh ({pos, normal}[nverts]) and uniform in
 // the grid box, each labelled with the trilinear value of the pose's grid (cells, truncated to
@@ -81,7 +96,6 @@ cudaError_t launch_init_params(float* params, uint32_t seed, __nv_bfloat16* wbf,
 cudaError_t launch_sample(const float4* mesh, int nverts, const float* grid, const SdfGrid& g, float band, float sigma,
                           float3 sphereCentre, float sphereRadius, Pose pose, int count, uint32_t seed, Sample* out,
                           cudaStream_t s);
-size_t acts_elements(int batch);
 
 // ---- the forward pass on the fifth-generation tensor cores (tcgen05, tfx_neural_tc.cu)
 // Packed weights: W1..W4 as K-major bf16 MMA operands [64 neurons][K] (K = 112 for layer 1, 80 for

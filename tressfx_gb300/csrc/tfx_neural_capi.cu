@@ -186,7 +186,7 @@ extern "C" int tfx_nsdf_train(tfx_nsdf h, int steps, int batch, float lr, float*
         if (h->acts) cudaFree(h->acts);
         h->acts = nullptr;
         h->actsBatch = 0;
-        TFX_CUDA(cudaMalloc(&h->acts, sizeof(__nv_bfloat16) * nsdf::acts_elements(batch)), "tfx_nsdf_train: activations");
+        TFX_CUDA(cudaMalloc(&h->acts, nsdf::train_scratch_bytes(batch)), "tfx_nsdf_train: activations");
         h->actsBatch = batch;
     }
     TFX_CUDA(cudaMemsetAsync(h->lossSum, 0, sizeof(float), s), "tfx_nsdf_train: loss");
@@ -194,12 +194,12 @@ extern "C" int tfx_nsdf_train(tfx_nsdf h, int steps, int batch, float lr, float*
     for (int k = 0; k < steps; ++k) {
         if (k == steps - tail) TFX_CUDA(cudaMemsetAsync(h->lossSum, 0, sizeof(float), s), "tfx_nsdf_train: loss");
         ++h->step;
-        cudaError_t e = nsdf::launch_train_step(h->wbf, h->bias, h->fr, h->pool[0], h->poolSize[0], batch,
-                                                h->seed * 2654435761u + (uint32_t)h->step * 40503u, h->acts, h->grads,
-                                                h->lossSum, s);
         // cosine decay of the learning rate over this call's steps, to a tenth of it
         const float lrk = lr * (0.1f + 0.45f * (1.0f + cosf(3.14159265f * (float)k / (float)steps)));
-        if (e == cudaSuccess) e = nsdf::launch_adam(h->params, h->grads, h->m, h->v, h->step, lrk, 1.0f, h->wbf, h->bias, s);
+        const cudaError_t e = nsdf::launch_train_step(
+            nsdf::TrainStep{h->wbf, h->bias, h->fr, h->pool[0], h->poolSize[0], batch,
+                            h->seed * 2654435761u + (uint32_t)h->step * 40503u, h->acts, h->params, h->grads, h->m, h->v,
+                            h->lossSum, h->step, lrk, k == 0 || k == steps - tail}, s);
         if (e != cudaSuccess) return cuda_fail(e, "tfx_nsdf_train: step launch");
     }
     if (cudaError_t e = nsdf::launch_pack_tc(h->params, h->wtc, s)) return cuda_fail(e, "tfx_nsdf_train: pack");
@@ -334,7 +334,7 @@ extern "C" int tfx_nsdf_set_params(tfx_nsdf h, const float* host, size_t count) 
     TFX_CUDA(cudaMemsetAsync(h->m, 0, sizeof(float) * count, s), "tfx_nsdf_set_params");
     TFX_CUDA(cudaMemsetAsync(h->v, 0, sizeof(float) * count, s), "tfx_nsdf_set_params");
     TFX_CUDA(cudaMemsetAsync(h->wbf, 0, sizeof(__nv_bfloat16) * nsdf::WBF_ALL, s), "tfx_nsdf_set_params");
-    cudaError_t e = nsdf::launch_adam(h->params, nullptr, nullptr, nullptr, 0, 0.f, 0.f, h->wbf, h->bias, s);
+    cudaError_t e = nsdf::launch_publish(h->params, h->wbf, h->bias, s);
     if (e == cudaSuccess) e = nsdf::launch_pack_tc(h->params, h->wtc, s);
     if (e != cudaSuccess) return cuda_fail(e, "tfx_nsdf_set_params");
     h->step = 0;
