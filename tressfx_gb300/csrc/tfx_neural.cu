@@ -7,7 +7,6 @@
 // C (16 x 8, f32) {row g, cols 2i, 2i+1}, {row g+8, cols 2i, 2i+1}.  The C fragments of n-tiles 2k and
 // 2k+1 are exactly the A fragment of k-tile k of the next layer, so activations never leave registers.
 #include <algorithm>
-#include <cmath>
 #include <type_traits>
 
 #include "tfx_launch.cuh"
@@ -302,6 +301,10 @@ __global__ void __launch_bounds__(QUERY_WARPS * 32) k_nsdf_query(const __nv_bflo
 }
 
 // ------------------------------------------------------------------------------------------ training
+__device__ __forceinline__ void copy_async16(void* dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
 // One minibatch: forward with saved activations, loss, backward to every layer's pre-activation
 // gradient.  Activations and gradients go to `acts` in the pair layout for k_nsdf_wgrad:
 //   H0 [B/2][KIN], H1..H4 [B/2][64], dZ1..dZ4 [B/2][64], dZ5 [B/2][8]   (32-bit words).
@@ -311,10 +314,6 @@ __global__ void __launch_bounds__(QUERY_WARPS * 32) k_nsdf_query(const __nv_bflo
 // on an SM and its time was one warp's chain through the ten layers.  A layer's activations pass between
 // the warps through shared memory (bf16, two buffers by turns), its pre-activations stay in registers for
 // the backward pass.  Bound: that chain and the barrier per layer (8,192 samples, ncu: 23.4 -> 11.9 us).
-__device__ __forceinline__ void copy_async16(void* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
-
 __device__ __forceinline__ void tile_sync(int tile) { asm volatile("bar.sync %0, 128;" ::"r"(tile + 1) : "memory"); }
 
 // Two n-tiles' words (bf16 pairs of columns c0, c0 + 1; [nt][0] row g, [nt][1] row g + 8) into the tile's
@@ -662,18 +661,20 @@ __global__ void k_nsdf_publish(const float* __restrict__ params, __nv_bfloat16* 
 
 // The gradient as the sum of its `nparts` parts, Adam (Kingma & Ba 2015) on the fp32 master parameters, then
 // their copies.  Eight lanes share four consecutive parameters: each adds an eighth of the parts, the first
-// four update one parameter each.  corr1, corr2: 1 - b1^step and 1 - b2^step.
+// four update one parameter each.
 constexpr int ADAM_THREADS = 256;
 static_assert(NPARAM % 4 == 0, "parameters are summed four at a time");
 __global__ void __launch_bounds__(ADAM_THREADS) k_nsdf_adam(float* __restrict__ params, const float* __restrict__ parts, int nparts,
                                                             float* __restrict__ grads, float* __restrict__ m, float* __restrict__ v,
-                                                            float corr1, float corr2, float lr, __nv_bfloat16* __restrict__ wbf,
+                                                            int step, float lr, __nv_bfloat16* __restrict__ wbf,
                                                             float* __restrict__ bias) {
     const int t = blockIdx.x * ADAM_THREADS + threadIdx.x;
     const int quad = t >> 3, lane8 = t & 7;
     const bool mine = quad < NPARAM / 4, update = mine && lane8 < 4;
     const int p = 4 * quad + lane8;
     // written by the step before, which ended before the launches this one follows began
+    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+    const float corr1 = 1.0f - powf(b1, (float)step), corr2 = 1.0f - powf(b2, (float)step);
     const float m0 = update ? m[p] : 0.f, v0 = update ? v[p] : 0.f, w0 = update ? params[p] : 0.f;
     after_previous();
     let_next_in();
@@ -694,7 +695,6 @@ __global__ void __launch_bounds__(ADAM_THREADS) k_nsdf_adam(float* __restrict__ 
     if (!update) return;
     const float g = lane8 == 0 ? gr.x : lane8 == 1 ? gr.y : lane8 == 2 ? gr.z : gr.w;
     grads[p] = g;
-    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     const float mm = b1 * m0 + (1.0f - b1) * g;
     const float vv = b2 * v0 + (1.0f - b2) * g * g;
     m[p] = mm; v[p] = vv;
@@ -807,10 +807,8 @@ cudaError_t launch_train_step(const TrainStep& t, cudaStream_t s) {
     const int chunks = t.batch / WG_SAMPLES, rounds = (chunks + TRAIN_PARTS - 1) / TRAIN_PARTS, nparts = (chunks + rounds - 1) / rounds;
     e = launch_after(k_nsdf_wgrad, (unsigned)nparts * 5, WG_THREADS, WG_SMEM, s, acts, t.batch, rounds, parts);
     if (e != cudaSuccess) return e;
-    const float corr1 = (float)(1.0 - std::pow((double)0.9f, (double)t.step));
-    const float corr2 = (float)(1.0 - std::pow((double)0.999f, (double)t.step));
     return launch_after(k_nsdf_adam, (NPARAM / 4 * 8 + ADAM_THREADS - 1) / ADAM_THREADS, ADAM_THREADS, 0, s, t.params, parts, nparts,
-                        t.grads, t.m, t.v, corr1, corr2, t.lr, t.wbf, t.bias);
+                        t.grads, t.m, t.v, t.step, t.lr, t.wbf, t.bias);
 }
 
 cudaError_t launch_publish(const float* params, __nv_bfloat16* wbf, float* bias, cudaStream_t s) {
