@@ -72,9 +72,10 @@ struct FusedLaunch {
     const BatchObject* objs;
     const WorkItem* items;
     int numItems;
-    int* err;        // set to 1 when a block gives up waiting for its bulk copies
+    int* err;        // page-locked host word, set to 1 when a block gives up waiting for its bulk copies
     int mode;        // 0 the whole frame, 1 up to the local-shape sweeps, 2 after them
     int waitPolls;   // limit of the first wait (kFusedWaitPollsDefault; 0 in tests of the timeout path)
+    bool after;      // the launch before it on the stream is a kernel it alone depends on (launch_after)
 };
 
 struct FollowLaunch {
@@ -95,6 +96,7 @@ struct SdfBatchLaunch {
     int constructThreads;
     TriJob* jobs;         // [totalTris]: written by the initialisation, read by the construct; null when the
                           // construct makes its own (sdf_takes_jobs)
+    bool after;      // the launch before it on the stream is a kernel it alone depends on (launch_after)
     int expand;      // some SDF keeps a corner-expanded copy: run the expansion
     // the SDFs that keep one, so that the expansion runs over their cells only: their indices into
     // `sdfs`, the prefix of their cell counts (nexp + 1 entries), and the sum

@@ -32,7 +32,7 @@ using namespace tfx;
 struct BatchClass {
     int n = 0;
     int vpl = 2, warps = 4, blocks = 1;
-    int perSMCap = 0;            // resident strand blocks per SM allowed (0 = as many as fit)
+    int perSMCap = 0;            // resident strand blocks per SM, persistent over the groups (0: a block per group)
     int followBlocks = 1;        // grid of k_follow_collide (persistent over the chunks)
     int followChunks = 1;        // chunks per group in k_follow_collide
     int followMode = 0;          // FollowLaunch::queued.  Default, from measurements: 1 when an object of the
@@ -40,6 +40,7 @@ struct BatchClass {
                                  // reach both surface and far vertices), else 0; the autotuner tries the others
     bool splitSweeps = false;    // local-shape sweeps in k_local_sweep between two strand passes
     bool noFollow = false;       // no object of the class has follow hairs
+    bool followWork = true;      // some object of the class has follow hairs or an SDF
     std::vector<WorkItem> hostItems;
     WorkItem* items = nullptr;  // device
     int numItems = 0;
@@ -73,6 +74,7 @@ struct tfx_batch_t {
     // already queued leaves the GPU busy
     char* pinned[kFrameSlots] = {};
     char* devBlock = nullptr;
+    bool uploadKernel = true;   // the frame block is brought over by a kernel (launch_upload), not the copy engine
     cudaEvent_t done[kFrameSlots] = {};
     bool used[kFrameSlots] = {};
     int slot = 0;
@@ -102,8 +104,10 @@ struct tfx_batch_t {
     // classes touch disjoint objects), so one class's last blocks run beside the next class's
     cudaStream_t classStream[5] = {};
     cudaEvent_t evClasses = nullptr, evClassDone[5] = {};
-    int* devErr = nullptr;      // fused kernel: a block gave up waiting for its bulk copies
-    int* pinnedErr = nullptr;   // its copy at the end of each frame, one word per slot
+    // strand kernel: a block gave up waiting for its bulk copies.  Page-locked words the kernel writes itself:
+    // one per frame slot, one for frames launched directly
+    int* pinnedErr = nullptr;
+    int errSlot = kFrameSlots;  // the word of the frame being launched or captured
     int waitPolls = kFusedWaitPollsDefault;   // TFX_BATCH_WAIT_POLLS
 
     cudaGraphExec_t graph[kFrameSlots] = {};
@@ -125,15 +129,14 @@ struct tfx_batch_t {
 static int batch_fail_built(const char* who) { return fail(TFX_ERR_INVALID_ARGUMENT, "%s: the batch is already built", who); }
 
 // A frame's fused strand kernel gave up waiting for its bulk copies: waits for the frames queued so
-// far, clears the device flag and both frames' copies of it (so the report is made once), and
+// far, clears every frame's flag (so the report is made once), and
 // returns TFX_ERR_TIMEOUT.  The state of the failed frame is undefined; the caller restores it
 // (tfx_hair_write) or resets the objects.
 static int report_timeout(tfx_batch b) {
     cudaSetDevice(b->ctx->device);
     cudaError_t e = cudaStreamSynchronize(b->ctx->stream);
-    if (e == cudaSuccess) e = cudaMemset(b->devErr, 0, sizeof(int));
     if (e != cudaSuccess) return cuda_fail(e, "tfx_batch: clearing the error flag");
-    for (int i = 0; i < kFrameSlots; ++i) b->pinnedErr[i] = 0;
+    for (int i = 0; i <= kFrameSlots; ++i) b->pinnedErr[i] = 0;
     return fail(TFX_ERR_TIMEOUT, "tfx_batch: a fused strand block gave up waiting for its bulk copies");
 }
 
@@ -272,10 +275,12 @@ static void make_items(tfx_batch b, BatchClass& c) {
     c.hostItems.clear();
     c.followMode = c.n >= 64 ? 2 : 0;
     c.noFollow = true;
+    c.followWork = false;
     for (int o = 0; o < (int)b->hairs.size(); ++o) {
         tfx_hair h = b->hairs[o];
         if (h->n != c.n) continue;
         if (h->F > 0) { c.followMode = 1; c.noFollow = false; }
+        if (h->F > 0 || b->hairSdf[o] >= 0) c.followWork = true;
         const int gsz = fused_group_size(c.n);
         for (int g = 0; g < h->G; g += gsz) c.hostItems.push_back(WorkItem{o, g, std::min(gsz, h->G - g), 0});
     }
@@ -291,13 +296,14 @@ static int upload_items(BatchClass& c) {
     return TFX_OK;
 }
 
-// Grid of a fused class: as many resident blocks as fit (persistent), no more than groups.
+// Grid of a fused class: a block per group, or, with a cap on the resident blocks, that many, each taking groups
+// in turn.  Blocks that end with their group let the concurrent kernels in as they end, and leave no
+// last round: the 200,000 x 16 frame went from 297 to 281 us.
 static int size_class(tfx_batch b, BatchClass& c) {
     int perSM = fused_blocks_per_sm(c.n, c.vpl, c.warps);
     if (perSM <= 0)
         return fail(TFX_ERR_CUDA, "tfx_batch: fused kernel n=%d vpl=%d with %d warps cannot be resident", c.n, c.vpl, c.warps);
-    if (c.perSMCap > 0) perSM = std::min(perSM, c.perSMCap);
-    c.blocks = std::max(1, std::min(perSM * b->ctx->numSMs, c.numItems));
+    c.blocks = std::max(1, c.perSMCap > 0 ? std::min(std::min(perSM, c.perSMCap) * b->ctx->numSMs, c.numItems) : c.numItems);
     // follow/collide: whole groups when every resident block gets at least four, else the smallest chunks
     const int fResident = std::max(1, follow_blocks_per_sm(c.n, c.followMode, c.noFollow)) * b->ctx->numSMs;
     c.followChunks = c.numItems >= 4 * fResident ? 1 : follow_max_chunks_per_item(c.n);
@@ -323,8 +329,8 @@ static int launch_sdf_part(tfx_batch b, cudaStream_t s) {
     return TFX_OK;
 }
 
-static int launch_strands(tfx_batch b, BatchClass& c, cudaStream_t s) {
-    FusedLaunch fl{c.n, c.vpl, c.warps, c.blocks, b->objTable, c.items, c.numItems, b->devErr, 0, b->waitPolls};
+static int launch_strands(tfx_batch b, BatchClass& c, cudaStream_t s, bool after) {
+    FusedLaunch fl{c.n, c.vpl, c.warps, c.blocks, b->objTable, c.items, c.numItems, b->pinnedErr + b->errSlot, 0, b->waitPolls, after};
     cudaError_t e;
     if (!c.splitSweeps) {
         e = launch_fused_strands(fl, s);
@@ -333,12 +339,14 @@ static int launch_strands(tfx_batch b, BatchClass& c, cudaStream_t s) {
         e = launch_fused_strands(fl, s);
         if (e == cudaSuccess) e = launch_local_sweep(fl, s);
         fl.mode = 2;
+        fl.after = true;
         if (e == cudaSuccess) e = launch_fused_strands(fl, s);
     }
     return e == cudaSuccess ? TFX_OK : cuda_fail(e, "tfx_batch: fused strand launch");
 }
 
 static int launch_follows(tfx_batch b, BatchClass& c, cudaStream_t s) {
+    if (!c.followWork) return TFX_OK;
     FollowLaunch fl{c.n, c.followBlocks, b->objTable, c.items, c.numItems, c.followChunks, c.followMode,
                     c.noFollow ? 1 : 0};
     cudaError_t e = launch_follow_collide(fl, s);
@@ -367,12 +375,13 @@ static int launch_frame_direct(tfx_batch b, cudaStream_t s, std::vector<float>* 
         cudaEventRecord(e, s);
         ev.push_back(e);
     };
+    b->errSlot = kFrameSlots;
     mark();
     if (int r = launch_sdf_part(b, s)) return r;
     mark();
     for (auto& c : b->classes) {
         if (c.numItems == 0) continue;
-        if (int r = launch_strands(b, c, s)) return r;
+        if (int r = launch_strands(b, c, s, false)) return r;
         mark();
     }
     for (auto& c : b->classes) {
@@ -386,9 +395,7 @@ static int launch_frame_direct(tfx_batch b, cudaStream_t s, std::vector<float>* 
     }
     if (partMs) {
         cudaEventSynchronize(ev.back());
-        int flag = 0;
-        cudaMemcpy(&flag, b->devErr, sizeof(int), cudaMemcpyDeviceToHost);
-        if (flag) {
+        if (*static_cast<volatile int*>(b->pinnedErr + kFrameSlots)) {
             for (auto e : ev) cudaEventDestroy(e);
             return report_timeout(b);
         }
@@ -420,7 +427,7 @@ static int launch_frame_forked(tfx_batch b, cudaStream_t s) {
     if (!b->overlap) {
         for (auto& c : b->classes)
             if (c.numItems > 0)
-                if (int r = launch_strands(b, c, s)) return r;
+                if (int r = launch_strands(b, c, s, false)) return r;
         for (auto& c : b->classes)
             if (c.numItems > 0)
                 if (int r = launch_follows(b, c, s)) return r;
@@ -432,7 +439,7 @@ static int launch_frame_forked(tfx_batch b, cudaStream_t s) {
         if (c.numItems == 0) continue;
         cudaStream_t cs = k == 0 ? s : b->classStream[k];
         if (k > 0) TFX_CUDA(cudaStreamWaitEvent(cs, b->evClasses, 0), "tfx_batch: class fork");
-        if (int r = launch_strands(b, c, cs)) return r;
+        if (int r = launch_strands(b, c, cs, k == 0 && b->uploadKernel)) return r;   // the first straight after the upload
         if (fork) TFX_CUDA(cudaStreamWaitEvent(cs, b->evJoin, 0), "tfx_batch: join");
         if (int r = launch_follows(b, c, cs)) return r;
         if (k > 0) TFX_CUDA(cudaEventRecord(b->evClassDone[k], cs), "tfx_batch: class join");
@@ -449,14 +456,12 @@ static int capture_graphs(tfx_batch b) {
         if (b->graph[slot]) { cudaGraphExecDestroy(b->graph[slot]); b->graph[slot] = nullptr; }
         cudaGraph_t g = nullptr;
         TFX_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
-        cudaError_t e = cudaMemcpyAsync(b->devBlock, b->pinned[slot], b->blockBytes, cudaMemcpyHostToDevice, s);
+        b->errSlot = slot;
+        cudaError_t e = b->uploadKernel ? launch_upload(b->devBlock, b->pinned[slot], b->blockBytes, s)
+                                        : cudaMemcpyAsync(b->devBlock, b->pinned[slot], b->blockBytes, cudaMemcpyHostToDevice, s);
         int r = TFX_OK;
         if (e != cudaSuccess) r = cuda_fail(e, "tfx_batch: capture upload");
         if (r == TFX_OK) r = launch_frame_forked(b, s);
-        if (r == TFX_OK) {
-            e = cudaMemcpyAsync(b->pinnedErr + slot, b->devErr, sizeof(int), cudaMemcpyDeviceToHost, s);
-            if (e != cudaSuccess) r = cuda_fail(e, "tfx_batch: capture error-flag copy");
-        }
         cudaError_t ee = cudaStreamEndCapture(s, &g);
         if (r != TFX_OK) { if (g) cudaGraphDestroy(g); return r; }
         if (ee != cudaSuccess) return cuda_fail(ee, "cudaStreamEndCapture");
@@ -470,7 +475,8 @@ static int capture_graphs(tfx_batch b) {
         else sdfLaunches = (b->sdfL.totalTris > 0 ? 3 : 2) + (b->sdfL.expand ? 1 : 0);
     }
     int launches = (b->totalMeshVerts > 0 ? 1 : 0) + sdfLaunches;
-    for (auto& c : b->classes) launches += c.numItems > 0 ? (c.splitSweeps ? 4 : 2) : 0;
+    for (auto& c : b->classes) launches += c.numItems > 0 ? (c.splitSweeps ? 3 : 1) + (c.followWork ? 1 : 0) : 0;
+    if (b->uploadKernel) ++launches;
     for (size_t k = 0; k < b->levelPairs.size(); ++k) launches += b->levelVertices[k] > 0 ? 1 : 0;
     b->launchesPerFrame = launches;
     return TFX_OK;
@@ -544,9 +550,7 @@ static int time_graph_frames(tfx_batch b, int frames, float* ms) {
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (e != cudaSuccess) return cuda_fail(e, "tfx_batch: autotune frames");
-    int flag = 0;
-    TFX_CUDA(cudaMemcpy(&flag, b->devErr, sizeof(int), cudaMemcpyDeviceToHost), "tfx_batch: error flag");
-    if (flag) return report_timeout(b);
+    if (*static_cast<volatile int*>(b->pinnedErr)) return report_timeout(b);
     *ms = best;
     return TFX_OK;
 }
@@ -736,9 +740,7 @@ extern "C" int tfx_batch_build(tfx_batch b, int reserved) {
     b->objTable = (BatchObject*)p; p += align256(sizes[0]);
     b->meshTable = (BatchMesh*)p; p += align256(sizes[1]);
     b->sdfTable = (BatchSdf*)p; p += align256(sizes[2]);
-    b->devErr = (int*)p;
-    TFX_CUDA(cudaMemset(b->devErr, 0, sizeof(int)), "tfx_batch: clear error flag");
-    TFX_CUDA(cudaMallocHost((void**)&b->pinnedErr, kFrameSlots * sizeof(int)), "tfx_batch: pinned error flag");
+    TFX_CUDA(cudaMallocHost((void**)&b->pinnedErr, (kFrameSlots + 1) * sizeof(int)), "tfx_batch: pinned error flags");
     TFX_CUDA(cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking), "tfx_batch: side stream");
     for (int i = 0; i < 5; ++i) {
         TFX_CUDA(cudaStreamCreateWithFlags(&b->classStream[i], cudaStreamNonBlocking), "tfx_batch: class stream");
@@ -747,7 +749,7 @@ extern "C" int tfx_batch_build(tfx_batch b, int reserved) {
     TFX_CUDA(cudaEventCreateWithFlags(&b->evClasses, cudaEventDisableTiming), "cudaEventCreate");
     TFX_CUDA(cudaEventCreateWithFlags(&b->evFork, cudaEventDisableTiming), "cudaEventCreate");
     TFX_CUDA(cudaEventCreateWithFlags(&b->evJoin, cudaEventDisableTiming), "cudaEventCreate");
-    for (int i = 0; i < kFrameSlots; ++i) b->pinnedErr[i] = 0;
+    for (int i = 0; i <= kFrameSlots; ++i) b->pinnedErr[i] = 0;
 
     // corner-expanded grids: 8 floats per cell, at the SDF's quad prefix
     std::vector<long long> sdfFirstQuad(nsdf, 0);
@@ -879,9 +881,23 @@ extern "C" int tfx_batch_build(tfx_batch b, int reserved) {
     if (sdf_takes_jobs(firstTri))
         TFX_CUDA(cudaMalloc(&b->jobArena, sdf_job_bytes() * (size_t)firstTri), "tfx_batch: triangle jobs");
     b->sdfL = SdfBatchLaunch{b->sdfTable, nsdf, firstTri, firstQuad, 128, reinterpret_cast<TriJob*>(b->jobArena),
-                             0, nullptr, nullptr, 0, 0};
+                             b->totalMeshVerts > 0, 0, nullptr, nullptr, 0, 0};
     b->expandMode = 2;
     if (int r = apply_expand_mode(b)) return r;
+
+    // How the frame block is brought over.  Between two frames of one stream a copy by the copy engine costs 5 us
+    // more than a kernel that reads the page-locked block itself (2,048 x 16 strands: 11.0 against 6.3 us a
+    // frame, a 2,240 x 32 character with follow hairs: 45 against 42).  But frames of several batches in flight
+    // then start in step, and where one frame's data alone passes the L2, they keep evicting one another's: three
+    // fur batches by turns take 332 us a frame with the kernel, 297 with the copy, three 16-object ones 748 and
+    // 730; at 180 MB (the film head) the kernel is ahead by 2 us.  The line is twice the L2.
+    {
+        double bytes = 0.0;   // what the strand and follow kernels read and write a frame
+        for (auto h : b->hairs) bytes += (132.0 + 36.0 * h->F) * h->G * h->n;
+        int l2 = 0;
+        TFX_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, b->ctx->device), "cudaDeviceGetAttribute");
+        b->uploadKernel = bytes <= 2.0 * l2;
+    }
 
     // ---- strand classes (one fused launch per vertices-per-strand count present)
     for (int n : {4, 8, 16, 32, 64}) {
@@ -978,7 +994,7 @@ static int claim_block(tfx_batch b, int* slotOut) {
     b->slot = (s + 1) % kFrameSlots;
     if (b->used[s]) {
         TFX_CUDA(cudaEventSynchronize(b->done[s]), "cudaEventSynchronize");
-        if (b->pinnedErr[s]) {
+        if (static_cast<volatile int*>(b->pinnedErr)[s]) {
             b->slot = s;   // the block stays unclaimed: the next call takes it
             return report_timeout(b);
         }
@@ -1004,7 +1020,7 @@ extern "C" int tfx_batch_synchronize(tfx_batch b) {
     TFX_CUDA(cudaSetDevice(b->ctx->device), "cudaSetDevice");
     TFX_CUDA(cudaStreamSynchronize(b->ctx->stream), "cudaStreamSynchronize");
     for (int s = 0; s < kFrameSlots; ++s)
-        if (b->used[s] && b->pinnedErr[s]) return report_timeout(b);
+        if (b->used[s] && static_cast<volatile int*>(b->pinnedErr)[s]) return report_timeout(b);
     return TFX_OK;
 }
 

@@ -36,6 +36,7 @@
 // plain path and the oracle bit for bit.
 #include "tfx_batch.h"
 #include "tfx_bulk.cuh"
+#include "tfx_launch.cuh"
 #include "tfx_sdf_math.cuh"
 
 namespace tfx {
@@ -44,6 +45,7 @@ namespace tfx {
 // collision-mesh skinning over all meshes
 __global__ void __launch_bounds__(256) k_batch_mesh_skin(const BatchMesh* __restrict__ meshes, int nmeshes,
                                                          int totalVerts) {
+    after_previous();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= totalVerts) return;
     int lo = 0, hi = nmeshes - 1;
@@ -93,6 +95,7 @@ __device__ __forceinline__ TriJob batch_job(const BatchSdf* __restrict__ sdfs, i
 // quad of an SDF may be partial), and with a job array the job of every triangle.
 __global__ void __launch_bounds__(256) k_batch_sdf_init(const BatchSdf* __restrict__ sdfs, int nsdf, long long totalQuads,
                                                         TriJob* __restrict__ jobs, int totalTris) {
+    after_previous();
     const uint32_t v = float_flip3(1e10f);
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < totalTris; t += stride)
@@ -113,6 +116,7 @@ __global__ void __launch_bounds__(256) k_batch_sdf_init(const BatchSdf* __restri
 // FinalizeSignedDistanceField, :400-412
 __global__ void __launch_bounds__(256) k_batch_sdf_finalize(const BatchSdf* __restrict__ sdfs, int nsdf,
                                                             long long totalQuads) {
+    after_previous();
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < totalQuads; q += stride) {
         const BatchSdf& s = sdfs[find_by_prefix_quad(sdfs, nsdf, q)];
@@ -138,6 +142,7 @@ __global__ void __launch_bounds__(256) k_batch_sdf_expand(const BatchSdf* __rest
                                                           const int* __restrict__ expSdf,
                                                           const long long* __restrict__ expFirst, int nexp,
                                                           long long expCells) {
+    after_previous();
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < expCells; t += stride) {
         int lo = 0, hi = nexp - 1;
@@ -165,6 +170,7 @@ __global__ void __launch_bounds__(256) k_batch_sdf_expand(const BatchSdf* __rest
 // one list).  WARPS = warps per block.
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? kConstructBlocksPerSM : 1) k_batch_sdf_construct(const TriJob* __restrict__ jobs, int totalTris) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char smem_sdf[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const SdfWarpArea area = sdf_warp_area(smem_sdf, warp, kSdfJobsAhead);
@@ -175,6 +181,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? kConstructBlocksPerSM
 // lane k making the job of the chunk's k-th.
 __global__ void __launch_bounds__(128) k_batch_sdf_construct_chunks(const BatchSdf* __restrict__ sdfs, int nsdf, int totalTris,
                                                                     int per) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char smem_sdf[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const SdfWarpArea area = sdf_warp_area(smem_sdf, warp, per);
@@ -348,6 +355,7 @@ template <int N, int VPL>
 __global__ void __launch_bounds__(256, N <= 16 ? 4 : (VPL <= 2 ? 3 : 2)) k_fused_strands(const BatchObject* __restrict__ objs,
                                                                         const WorkItem* __restrict__ items, int numItems,
                                                                         int* err, int mode, int waitPolls) {
+    after_previous();
     constexpr int GS = fused_group_strands(N);
     constexpr int RS = N + 1;       // tile row stride, float4
     constexpr int L = N / VPL;      // lanes per strand in the per-strand passes
@@ -409,7 +417,7 @@ __global__ void __launch_bounds__(256, N <= 16 ? 4 : (VPL <= 2 ? 3 : 2)) k_fused
         // as failed, and a bounded wait is preferred over one that could hang the device).
         const bool arrived = mbar_wait_bounded(bar, parity, waitPolls);
         if (__syncthreads_or(!arrived)) {
-            if (tid == 0) atomicOr(err, 1);
+            if (tid == 0) *reinterpret_cast<volatile int*>(err) = 1;
             mbar_wait_bounded(bar, parity, kFusedWaitPollsDefault);
             return;
         }
@@ -667,6 +675,7 @@ __device__ __forceinline__ float3 bind_pose(const HairView& h, size_t vg, Q4 bq,
 template <int N>
 __global__ void __launch_bounds__(128) k_local_sweep(const BatchObject* __restrict__ objs,
                                                      const WorkItem* __restrict__ items, int numItems) {
+    after_previous();
     constexpr int GS = fused_group_strands(N);
     constexpr int IPW = 32 / GS;     // work items per warp
     constexpr int KMAX = 4;
@@ -1072,6 +1081,9 @@ cudaError_t launch_snapshot_positions(const BatchObject* objs, const long long* 
 template <int N, int VPL>
 static cudaError_t launch_fused_nv(const FusedLaunch& fl, cudaStream_t s) {
     // the dynamic shared-memory attribute is set by fused_blocks_per_sm before the first launch
+    if (fl.after)
+        return launch_after(k_fused_strands<N, VPL>, fl.blocks, fl.warpsPerBlock * 32, fused_smem_for(N), s, fl.objs, fl.items,
+                            fl.numItems, fl.err, fl.mode, fl.waitPolls);
     k_fused_strands<N, VPL><<<fl.blocks, fl.warpsPerBlock * 32, fused_smem_for(N), s>>>(fl.objs, fl.items, fl.numItems,
                                                                                         fl.err, fl.mode, fl.waitPolls);
     return cudaGetLastError();
@@ -1091,8 +1103,7 @@ template <int N>
 static cudaError_t launch_sweep_n(const FusedLaunch& fl, cudaStream_t s) {
     constexpr int IPW = 32 / fused_group_strands(N);
     const long long threads = (long long)((fl.numItems + IPW - 1) / IPW) * 32;
-    k_local_sweep<N><<<(unsigned)((threads + 127) / 128), 128, 0, s>>>(fl.objs, fl.items, fl.numItems);
-    return cudaGetLastError();
+    return launch_after(k_local_sweep<N>, (unsigned)((threads + 127) / 128), 128, 0, s, fl.objs, fl.items, fl.numItems);
 }
 
 cudaError_t launch_local_sweep(const FusedLaunch& fl, cudaStream_t s) {
@@ -1270,31 +1281,37 @@ cudaError_t launch_batch_sdf(const SdfBatchLaunch& L, cudaStream_t s) {
     const unsigned gq = (unsigned)std::min<long long>((q + 255) / 256, (long long)sm_count() * 32);
     const long long initWork = std::max<long long>(q, L.jobs ? L.totalTris : 0);
     const unsigned gi = (unsigned)std::min<long long>((initWork + 255) / 256, (long long)sm_count() * 32);
-    k_batch_sdf_init<<<gi, 256, 0, s>>>(L.sdfs, L.nsdf, q, L.jobs, L.jobs ? L.totalTris : 0);
+    const int njobs = L.jobs ? L.totalTris : 0;
+    cudaError_t e = cudaSuccess;
+    if (L.after) {
+        e = launch_after(k_batch_sdf_init, gi, 256, 0, s, L.sdfs, L.nsdf, q, L.jobs, njobs);
+    } else {
+        k_batch_sdf_init<<<gi, 256, 0, s>>>(L.sdfs, L.nsdf, q, L.jobs, njobs);
+        e = cudaGetLastError();
+    }
+    if (e != cudaSuccess) return e;
     if (L.totalTris > 0 && L.jobs) {
         const int wpb = L.constructThreads / 32;
         const size_t smem = sdf_construct_smem(wpb, kSdfJobsAhead);
         const unsigned blocks = (unsigned)std::min<long long>(((long long)L.totalTris + wpb - 1) / wpb,
                                                               (long long)sm_count() * sdf_construct_blocks_per_sm(L.constructThreads));
-        if (wpb == 2) k_batch_sdf_construct<2><<<blocks, 64, smem, s>>>(L.jobs, L.totalTris);
-        else if (wpb == 8) k_batch_sdf_construct<8><<<blocks, 256, smem, s>>>(L.jobs, L.totalTris);
-        else k_batch_sdf_construct<4><<<blocks, 128, smem, s>>>(L.jobs, L.totalTris);
+        e = launch_after(wpb == 2 ? k_batch_sdf_construct<2> : wpb == 8 ? k_batch_sdf_construct<8> : k_batch_sdf_construct<4>, blocks,
+                         32 * wpb, smem, s, static_cast<const TriJob*>(L.jobs), L.totalTris);
     } else if (L.totalTris > 0) {
         const int per = sdf_construct_chunk(L.totalTris, sm_count());
         const long long chunks = ((long long)L.totalTris + per - 1) / per;
         const unsigned blocks = (unsigned)std::min<long long>((chunks + 3) / 4, (long long)sm_count() * 64);
-        k_batch_sdf_construct_chunks<<<blocks, 128, sdf_construct_smem(4, per), s>>>(L.sdfs, L.nsdf, L.totalTris, per);
+        e = launch_after(k_batch_sdf_construct_chunks, blocks, 128, sdf_construct_smem(4, per), s, L.sdfs, L.nsdf, L.totalTris, per);
     }
-    k_batch_sdf_finalize<<<gq, 256, 0, s>>>(L.sdfs, L.nsdf, q);
-    if (L.expand) return launch_batch_sdf_expand(L, s);
-    return cudaGetLastError();
+    if (e == cudaSuccess) e = launch_after(k_batch_sdf_finalize, gq, 256, 0, s, L.sdfs, L.nsdf, q);
+    if (e != cudaSuccess || !L.expand) return e;
+    return launch_batch_sdf_expand(L, s);
 }
 
 cudaError_t launch_batch_sdf_expand(const SdfBatchLaunch& L, cudaStream_t s) {
     if (L.nsdf <= 0 || !L.expand || L.expCells <= 0) return cudaSuccess;
     const unsigned ge = (unsigned)std::min<long long>((L.expCells + 255) / 256, (long long)sm_count() * 32);
-    k_batch_sdf_expand<<<ge, 256, 0, s>>>(L.sdfs, L.expSdf, L.expFirst, L.nexp, L.expCells);
-    return cudaGetLastError();
+    return launch_after(k_batch_sdf_expand, ge, 256, 0, s, L.sdfs, L.expSdf, L.expFirst, L.nexp, L.expCells);
 }
 
 }  // namespace tfx

@@ -318,7 +318,7 @@ extern "C" int tfx_hair_update_constants(tfx_hair h, const tfx_sim_params* p, in
     std::memcpy(c->bones, p->bone_matrices, (size_t)num_bones * 64);
     const size_t bytes = offsetof(DevSimConsts, bones) + (size_t)num_bones * 64;
     TFX_CUDA(cudaSetDevice(h->ctx->device), "cudaSetDevice");
-    TFX_CUDA(cudaMemcpyAsync(h->consts, c, bytes, cudaMemcpyHostToDevice, h->ctx->stream), "tfx_hair_update_constants: copy");
+    TFX_CUDA(launch_upload(h->consts, c, bytes, h->ctx->stream), "tfx_hair_update_constants: copy");
     TFX_CUDA(cudaEventRecord(h->stagingDone[slot], h->ctx->stream), "cudaEventRecord");
     h->stagingUsed[slot] = true;
     return TFX_OK;
@@ -651,8 +651,7 @@ extern "C" int tfx_mesh_skin(tfx_mesh m, const float* bone_matrices, int num_bon
         m->stagingNext ^= 1;
         if (m->stagingUsed[slot]) TFX_CUDA(cudaEventSynchronize(m->stagingDone[slot]), "cudaEventSynchronize");
         std::memcpy(m->staging[slot], bone_matrices, 64 * (size_t)num_bones);
-        TFX_CUDA(cudaMemcpyAsync(m->bones, m->staging[slot], 64 * (size_t)num_bones, cudaMemcpyHostToDevice, m->ctx->stream),
-                 "tfx_mesh_skin: bone upload");
+        TFX_CUDA(launch_upload(m->bones, m->staging[slot], 64 * (size_t)num_bones, m->ctx->stream), "tfx_mesh_skin: bone upload");
         TFX_CUDA(cudaEventRecord(m->stagingDone[slot], m->ctx->stream), "cudaEventRecord");
         m->stagingUsed[slot] = true;
     }

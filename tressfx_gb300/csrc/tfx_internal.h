@@ -47,6 +47,9 @@ struct SdfGrid {
 // launches size their grids as a multiple of it.
 int sm_count();
 
+// `bytes` (a multiple of 16) of page-locked host memory to the device, in stream order.
+cudaError_t launch_upload(void* dst, const void* pinned, size_t bytes, cudaStream_t s);
+
 // Launchers (tfx_sim_kernels.cu / tfx_sdf_kernels.cu). Return cudaGetLastError() of the launch.
 cudaError_t launch_integrate(const HairView& h, cudaStream_t s);
 cudaError_t launch_strand_level(const HairView& h, cudaStream_t s);

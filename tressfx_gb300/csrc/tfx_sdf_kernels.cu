@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <atomic>
 
+#include "tfx_launch.cuh"
 #include "tfx_sdf_math.cuh"
 
 namespace tfx {
@@ -26,6 +27,7 @@ __device__ __forceinline__ TriJob plain_job(uint32_t* sdf, const SdfGrid& g, con
 __global__ void __launch_bounds__(256) k_sdf_initialize(uint32_t* __restrict__ sdf, long long cells, SdfGrid g,
                                                         const float4* __restrict__ mesh, const uint32_t* __restrict__ idx,
                                                         int ntri, TriJob* __restrict__ jobs) {
+    after_previous();
     const uint32_t v = float_flip3(1e10f);
     const long long n4 = cells >> 2;
     const long long stride = (long long)gridDim.x * blockDim.x;
@@ -38,6 +40,7 @@ __global__ void __launch_bounds__(256) k_sdf_initialize(uint32_t* __restrict__ s
 
 // ConstructSignedDistanceField, :329-397, over the jobs made beforehand.
 __global__ void __launch_bounds__(128, kConstructBlocksPerSM) k_sdf_construct_jobs(const TriJob* __restrict__ jobs, int ntri) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const SdfWarpArea area = sdf_warp_area(smem, warp, kSdfJobsAhead);
@@ -50,6 +53,7 @@ __global__ void __launch_bounds__(128, kConstructBlocksPerSM) k_sdf_construct_jo
 __global__ void __launch_bounds__(128) k_sdf_construct(uint32_t* __restrict__ sdf, SdfGrid g,
                                                        const float4* __restrict__ mesh,
                                                        const uint32_t* __restrict__ idx, int ntri, int per) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     SdfWarpArea area = sdf_warp_area(smem, warp, per);
@@ -65,6 +69,7 @@ __global__ void __launch_bounds__(128) k_sdf_construct(uint32_t* __restrict__ sd
 
 // FinalizeSignedDistanceField, :400-412 (vectorised)
 __global__ void __launch_bounds__(256) k_sdf_finalize(uint32_t* __restrict__ sdf, long long cells) {
+    after_previous();
     const long long n4 = cells >> 2;
     const long long stride = (long long)gridDim.x * blockDim.x;
     uint4* s4 = reinterpret_cast<uint4*>(sdf);
@@ -80,6 +85,7 @@ __global__ void __launch_bounds__(256) k_sdf_finalize(uint32_t* __restrict__ sdf
 __global__ void __launch_bounds__(256) k_sdf_collide(const float* __restrict__ sdf, SdfGrid g, float margin,
                                                      float4* __restrict__ pos, float4* __restrict__ prev,
                                                      int n, long long vtot) {
+    after_previous();
     const long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (v >= vtot) return;
     const int local = (int)(v % n);
@@ -111,6 +117,7 @@ __global__ void __launch_bounds__(256) k_sdf_collide(const float* __restrict__ s
 __global__ void __launch_bounds__(256) k_sdf_collide_mixed(const float* __restrict__ sdf, SdfGrid g, float margin,
                                                            float4* __restrict__ pos, float4* __restrict__ prev,
                                                            int64_t vtot) {
+    after_previous();
     const int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (v >= vtot) return;
     const float4 hv = pos[v];
@@ -149,6 +156,7 @@ __global__ void __launch_bounds__(256) k_sdf_collide_mixed(const float* __restri
 __global__ void __launch_bounds__(256) k_mesh_skin(float4* __restrict__ out, const float4* __restrict__ in,
                                                    const float4* __restrict__ skin, const float4* __restrict__ bones,
                                                    int nverts) {
+    after_previous();
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nverts) return;
     const float4 p = __ldg(in + 2 * v), nr = __ldg(in + 2 * v + 1);
@@ -156,6 +164,18 @@ __global__ void __launch_bounds__(256) k_mesh_skin(float4* __restrict__ out, con
     blend_bones(bones, __ldg(skin + 2 * v), __ldg(skin + 2 * v + 1), m);
     out[2 * v] = with_xyz(p, xform_row(xyz(p), 1.0f, m));
     out[2 * v + 1] = with_xyz(nr, xform_row(xyz(nr), 0.0f, m));
+}
+
+// A frame's inputs from page-locked host memory, read by the kernel itself: `quads` 16-byte words.  Between two
+// kernels a copy by the copy engine costs 7 us, this 2.
+__global__ void __launch_bounds__(128) k_upload(const uint4* src, uint4* __restrict__ dst, int quads) {
+    after_previous();
+    let_next_in();
+    for (int i = blockIdx.x * 128 + threadIdx.x; i < quads; i += gridDim.x * 128) {
+        uint4 v;
+        asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(src + i));
+        dst[i] = v;
+    }
 }
 
 // --------------------------------------------------------------------------------------------
@@ -181,27 +201,32 @@ static inline unsigned grid_for(long long work, int threads, unsigned cap) {
 size_t sdf_job_bytes() { return sizeof(TriJob); }
 bool sdf_takes_jobs(int64_t tris) { return sdf_wants_jobs(tris, sm_count()); }
 
+cudaError_t launch_upload(void* dst, const void* pinned, size_t bytes, cudaStream_t s) {
+    const int quads = (int)(bytes / 16);
+    if (quads <= 0) return cudaSuccess;
+    return launch_after(k_upload, grid_for(quads, 128, sm_count() * 4), 128, 0, s, static_cast<const uint4*>(pinned),
+                        static_cast<uint4*>(dst), quads);
+}
+
 cudaError_t launch_sdf_initialize(uint32_t* sdf, int64_t cells, cudaStream_t s, const SdfGrid* g, const float4* mesh,
                                   const uint32_t* idx, int ntri, TriJob* jobs) {
     if (cells <= 0) return cudaSuccess;
     const int n = jobs ? ntri : 0;
     const long long work = std::max<long long>((cells + 3) / 4, n);
-    k_sdf_initialize<<<grid_for(work, 256, sm_count() * 16), 256, 0, s>>>(sdf, cells, g ? *g : SdfGrid{}, mesh, idx, n, jobs);
-    return cudaGetLastError();
+    return launch_after(k_sdf_initialize, grid_for(work, 256, sm_count() * 16), 256, 0, s, sdf, cells, g ? *g : SdfGrid{}, mesh,
+                        idx, n, jobs);
 }
 
 cudaError_t launch_sdf_jobs(TriJob* jobs, uint32_t* sdf, const SdfGrid& g, const float4* mesh, const uint32_t* idx, int ntri,
                             cudaStream_t s) {
     if (ntri <= 0) return cudaSuccess;
-    k_sdf_initialize<<<grid_for(ntri, 256, sm_count() * 16), 256, 0, s>>>(sdf, 0, g, mesh, idx, ntri, jobs);
-    return cudaGetLastError();
+    return launch_after(k_sdf_initialize, grid_for(ntri, 256, sm_count() * 16), 256, 0, s, sdf, 0, g, mesh, idx, ntri, jobs);
 }
 
 cudaError_t launch_sdf_construct_jobs(const TriJob* jobs, int ntri, cudaStream_t s) {
     if (ntri <= 0) return cudaSuccess;
     const unsigned blocks = (unsigned)std::min<long long>(((long long)ntri + 3) / 4, (long long)sm_count() * kConstructBlocksPerSM);
-    k_sdf_construct_jobs<<<blocks, 128, sdf_construct_smem(4, kSdfJobsAhead), s>>>(jobs, ntri);
-    return cudaGetLastError();
+    return launch_after(k_sdf_construct_jobs, blocks, 128, sdf_construct_smem(4, kSdfJobsAhead), s, jobs, ntri);
 }
 
 cudaError_t launch_sdf_construct(uint32_t* sdf, const SdfGrid& g, const float4* mesh, const uint32_t* idx, int ntri,
@@ -210,37 +235,32 @@ cudaError_t launch_sdf_construct(uint32_t* sdf, const SdfGrid& g, const float4* 
     const int per = sdf_construct_chunk(ntri, sm_count());
     const long long chunks = ((long long)ntri + per - 1) / per;
     const unsigned blocks = (unsigned)std::min<long long>((chunks + 3) / 4, (long long)sm_count() * 64);
-    k_sdf_construct<<<blocks, 128, sdf_construct_smem(4, per), s>>>(sdf, g, mesh, idx, ntri, per);
-    return cudaGetLastError();
+    return launch_after(k_sdf_construct, blocks, 128, sdf_construct_smem(4, per), s, sdf, g, mesh, idx, ntri, per);
 }
 
 cudaError_t launch_sdf_finalize(uint32_t* sdf, int64_t cells, cudaStream_t s) {
     if (cells <= 0) return cudaSuccess;
-    k_sdf_finalize<<<grid_for((cells + 3) / 4, 256, sm_count() * 16), 256, 0, s>>>(sdf, cells);
-    return cudaGetLastError();
+    return launch_after(k_sdf_finalize, grid_for((cells + 3) / 4, 256, sm_count() * 16), 256, 0, s, sdf, cells);
 }
 
 cudaError_t launch_sdf_collide(const uint32_t* sdf, const SdfGrid& g, float margin, float4* pos, float4* prev, int n,
                                int64_t vtot, cudaStream_t s) {
     if (vtot <= 0) return cudaSuccess;
-    k_sdf_collide<<<(unsigned)((vtot + 255) / 256), 256, 0, s>>>(reinterpret_cast<const float*>(sdf), g, margin, pos,
-                                                                 prev, n, vtot);
-    return cudaGetLastError();
+    return launch_after(k_sdf_collide, (unsigned)((vtot + 255) / 256), 256, 0, s, reinterpret_cast<const float*>(sdf), g, margin,
+                        pos, prev, n, vtot);
 }
 
 cudaError_t launch_sdf_collide_mixed(const uint32_t* sdf, const SdfGrid& g, float margin, float4* pos, float4* prev,
                                      int64_t vtot, cudaStream_t s) {
     if (vtot <= 0) return cudaSuccess;
-    k_sdf_collide_mixed<<<(unsigned)((vtot + 255) / 256), 256, 0, s>>>(reinterpret_cast<const float*>(sdf), g, margin, pos,
-                                                                       prev, vtot);
-    return cudaGetLastError();
+    return launch_after(k_sdf_collide_mixed, (unsigned)((vtot + 255) / 256), 256, 0, s, reinterpret_cast<const float*>(sdf), g,
+                        margin, pos, prev, vtot);
 }
 
 cudaError_t launch_mesh_skin(float4* out, const float4* in, const float4* skin, const float4* bones, int nverts,
                              cudaStream_t s) {
     if (nverts <= 0) return cudaSuccess;
-    k_mesh_skin<<<(nverts + 255) / 256, 256, 0, s>>>(out, in, skin, bones, nverts);
-    return cudaGetLastError();
+    return launch_after(k_mesh_skin, (nverts + 255) / 256, 256, 0, s, out, in, skin, bones, nverts);
 }
 
 }  // namespace tfx

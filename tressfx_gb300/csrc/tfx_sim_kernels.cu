@@ -13,6 +13,7 @@
 // tfx_device_math.cuh), so results match the FP32 oracle bit for bit.
 #include "tfx_device_math.cuh"
 #include "tfx_internal.h"
+#include "tfx_launch.cuh"
 
 namespace tfx {
 
@@ -20,6 +21,7 @@ namespace tfx {
 // IntegrationAndGlobalShapeConstraints, TressFXSimulation.hlsl:609-666.  One thread per guide vertex.
 template <int N>
 __global__ void __launch_bounds__(256) k_integrate(HairView h) {
+    after_previous();
     const DevSimConsts* __restrict__ c = h.consts;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= h.G * N) return;
@@ -69,6 +71,7 @@ __global__ void __launch_bounds__(256) k_integrate(HairView h) {
 // --------------------------------------------------------------------------------------------
 // CalculateStrandLevelData, TressFXSimulation.hlsl:677-728.  One thread per guide strand.
 __global__ void __launch_bounds__(128) k_strand_level(HairView h) {
+    after_previous();
     const DevSimConsts* __restrict__ c = h.consts;
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= h.G) return;
@@ -104,6 +107,7 @@ __global__ void __launch_bounds__(128) k_strand_level(HairView h) {
 // VelocityShockPropagation, TressFXSimulation.hlsl:739-762.  One thread per guide vertex.
 template <int N>
 __global__ void __launch_bounds__(256) k_vsp(HairView h) {
+    after_previous();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= h.G * N) return;
     const int g = t / N, j = t % N;
@@ -129,6 +133,7 @@ __global__ void __launch_bounds__(256) k_vsp(HairView h) {
 // are staged in shared memory as [vertex][strand] rows padded to 33 entries.
 template <int N>
 __global__ void __launch_bounds__(32) k_local_shape(HairView h) {
+    after_previous();
     constexpr int S = 32, LD = S + 1;
     extern __shared__ float4 smem[];
     float4* P = smem;                        // [N][LD] positions
@@ -193,6 +198,7 @@ __global__ void __launch_bounds__(32) k_local_shape(HairView h) {
 
 template <int N>
 __global__ void __launch_bounds__(256) k_length_wind(HairView h) {
+    after_previous();
     constexpr int L = N < 32 ? N : 32;
     constexpr int VPL = N / L;
     constexpr int SPW = 32 / L;
@@ -319,6 +325,7 @@ __global__ void __launch_bounds__(256) k_length_wind(HairView h) {
 // UpdateFollowHairVertices, TressFXSimulation.hlsl:978-1001.  One thread per follow vertex.
 template <int N>
 __global__ void __launch_bounds__(256) k_follow(HairView h) {
+    after_previous();
     const DevSimConsts* __restrict__ c = h.consts;
     const int per = h.F * N;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -353,20 +360,19 @@ static inline unsigned blocks_for(long long work, int threads) { return (unsigne
 
 cudaError_t launch_integrate(const HairView& h, cudaStream_t s) {
     if (h.G <= 0) return cudaSuccess;
-    TFX_SWITCH_N(h.n, (k_integrate<NN><<<blocks_for((long long)h.G * NN, 256), 256, 0, s>>>(h)));
-    return cudaGetLastError();
+    TFX_SWITCH_N(h.n, return launch_after(k_integrate<NN>, blocks_for((long long)h.G * NN, 256), 256, 0, s, h));
+    return cudaSuccess;
 }
 
 cudaError_t launch_strand_level(const HairView& h, cudaStream_t s) {
     if (h.G <= 0) return cudaSuccess;
-    k_strand_level<<<blocks_for(h.G, 128), 128, 0, s>>>(h);
-    return cudaGetLastError();
+    return launch_after(k_strand_level, blocks_for(h.G, 128), 128, 0, s, h);
 }
 
 cudaError_t launch_vsp(const HairView& h, cudaStream_t s) {
     if (h.G <= 0) return cudaSuccess;
-    TFX_SWITCH_N(h.n, (k_vsp<NN><<<blocks_for((long long)h.G * NN, 256), 256, 0, s>>>(h)));
-    return cudaGetLastError();
+    TFX_SWITCH_N(h.n, return launch_after(k_vsp<NN>, blocks_for((long long)h.G * NN, 256), 256, 0, s, h));
+    return cudaSuccess;
 }
 
 template <int N>
@@ -378,8 +384,7 @@ static cudaError_t launch_local_shape_n(const HairView& h, cudaStream_t s) {
         if (e != cudaSuccess) return e;
         configured = true;
     }
-    k_local_shape<N><<<blocks_for(h.G, 32), 32, smem, s>>>(h);
-    return cudaGetLastError();
+    return launch_after(k_local_shape<N>, blocks_for(h.G, 32), 32, smem, s, h);
 }
 
 cudaError_t launch_local_shape(const HairView& h, cudaStream_t s) {
@@ -392,8 +397,7 @@ template <int N>
 static cudaError_t launch_length_wind_n(const HairView& h, cudaStream_t s) {
     constexpr int L = N < 32 ? N : 32;  // lanes per strand
     const long long lanes = (long long)((h.G + (32 / L) - 1) / (32 / L)) * 32;
-    k_length_wind<N><<<blocks_for(lanes, 256), 256, 0, s>>>(h);
-    return cudaGetLastError();
+    return launch_after(k_length_wind<N>, blocks_for(lanes, 256), 256, 0, s, h);
 }
 
 cudaError_t launch_length_wind(const HairView& h, cudaStream_t s) {
@@ -404,8 +408,8 @@ cudaError_t launch_length_wind(const HairView& h, cudaStream_t s) {
 
 cudaError_t launch_follow(const HairView& h, cudaStream_t s) {
     if (h.G <= 0 || h.F <= 0) return cudaSuccess;
-    TFX_SWITCH_N(h.n, (k_follow<NN><<<blocks_for((long long)h.G * h.F * NN, 256), 256, 0, s>>>(h)));
-    return cudaGetLastError();
+    TFX_SWITCH_N(h.n, return launch_after(k_follow<NN>, blocks_for((long long)h.G * h.F * NN, 256), 256, 0, s, h));
+    return cudaSuccess;
 }
 
 }  // namespace tfx
