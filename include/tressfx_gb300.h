@@ -375,12 +375,11 @@ typedef enum tfx_batch_option {
     TFX_BATCH_SPLIT_SWEEPS = 4,     /* 1: the local-shape sweeps run as their own launch (a thread per
                                        strand, up to four sweeps pipelined in registers) between two
                                        passes of the strand kernel; 0: inside the strand kernel      */
-    TFX_BATCH_FOLLOW_FORM = 5,      /* the follow-hair + collision kernel of every class: 0 one vertex
-                                       at a time per thread; 1 the vertices needing a lookup, then
-                                       those within the margin, queued per warp and processed 32 at
-                                       a time; 2 only the gradient stage queued.  Default per class:
-                                       1 with follow hairs, else 2 at n >= 64, else 0 (get_option
-                                       reports the first class's)                                   */
+    TFX_BATCH_FOLLOW_FORM = 5,      /* 0, 1 or 2: chose between forms of the follow-hair + collision
+                                       kernel.  One form is the fastest everywhere now and runs for
+                                       every value; the value is still checked, kept and reported
+                                       (get_option: the first class's; default 1 with follow hairs,
+                                       else 2 at n >= 64, else 0)                                    */
     TFX_BATCH_WAIT_POLLS = 6,       /* polls of the strand kernel's bounded wait for a group's bulk
                                        copies before its block gives up and the frame reports
                                        TFX_ERR_TIMEOUT (default 2^21; 0 gives up at once, for tests

@@ -35,9 +35,7 @@ struct BatchClass {
     int perSMCap = 0;            // resident strand blocks per SM, persistent over the groups (0: a block per group)
     int followBlocks = 1;        // grid of k_follow_collide (persistent over the chunks)
     int followChunks = 1;        // chunks per group in k_follow_collide
-    int followMode = 0;          // FollowLaunch::queued.  Default, from measurements: 1 when an object of the
-                                 // class has follow hairs, else 2 at n >= 64 (long strands: lanes of one warp
-                                 // reach both surface and far vertices), else 0; the autotuner tries the others
+    int followForm = 0;          // TFX_BATCH_FOLLOW_FORM as last set or as it defaults: kept, and read back
     bool splitSweeps = false;    // local-shape sweeps in k_local_sweep between two strand passes
     bool noFollow = false;       // no object of the class has follow hairs
     bool followWork = true;      // some object of the class has follow hairs or an SDF
@@ -261,11 +259,9 @@ static void describe(tfx_batch b) {
     int k = b->sdfForm == 1 ? snprintf(buf, sizeof(buf), "sdf construct on 8x8x4-cell tiles (a warp per 4x4x2 brick), %d blocks;", b->sdfT.blocks)
                             : snprintf(buf, sizeof(buf), "sdf construct %d threads/block;", b->sdfL.constructThreads);
     for (auto& c : b->classes)
-        k += snprintf(buf + k, sizeof(buf) - k, " n=%d: %d vertices/lane, %d warps/block, %d blocks, %d groups of %d%s%s;",
+        k += snprintf(buf + k, sizeof(buf) - k, " n=%d: %d vertices/lane, %d warps/block, %d blocks, %d groups of %d%s;",
                       c.n, c.vpl, c.warps, c.blocks, c.numItems, fused_group_size(c.n),
-                      c.splitSweeps ? ", sweeps in their own launch" : "",
-                      c.followMode == 1 ? ", collide on per-warp lookup queues"
-                                         : c.followMode == 2 ? ", gradient lookups on per-warp queues" : "");
+                      c.splitSweeps ? ", sweeps in their own launch" : "");
     k += snprintf(buf + k, sizeof(buf) - k, " SDF build %s the strand kernels%s;",
                   b->overlap ? "concurrent with" : "before", b->sdfL.expand ? ", lookups on corner-expanded grids" : "");
     b->description = buf;
@@ -273,13 +269,13 @@ static void describe(tfx_batch b) {
 
 static void make_items(tfx_batch b, BatchClass& c) {
     c.hostItems.clear();
-    c.followMode = c.n >= 64 ? 2 : 0;
+    c.followForm = c.n >= 64 ? 2 : 0;
     c.noFollow = true;
     c.followWork = false;
     for (int o = 0; o < (int)b->hairs.size(); ++o) {
         tfx_hair h = b->hairs[o];
         if (h->n != c.n) continue;
-        if (h->F > 0) { c.followMode = 1; c.noFollow = false; }
+        if (h->F > 0) { c.followForm = 1; c.noFollow = false; }
         if (h->F > 0 || b->hairSdf[o] >= 0) c.followWork = true;
         const int gsz = fused_group_size(c.n);
         for (int g = 0; g < h->G; g += gsz) c.hostItems.push_back(WorkItem{o, g, std::min(gsz, h->G - g), 0});
@@ -305,7 +301,7 @@ static int size_class(tfx_batch b, BatchClass& c) {
         return fail(TFX_ERR_CUDA, "tfx_batch: fused kernel n=%d vpl=%d with %d warps cannot be resident", c.n, c.vpl, c.warps);
     c.blocks = std::max(1, c.perSMCap > 0 ? std::min(std::min(perSM, c.perSMCap) * b->ctx->numSMs, c.numItems) : c.numItems);
     // follow/collide: whole groups when every resident block gets at least four, else the smallest chunks
-    const int fResident = std::max(1, follow_blocks_per_sm(c.n, c.followMode, c.noFollow)) * b->ctx->numSMs;
+    const int fResident = std::max(1, follow_blocks_per_sm(c.n, c.noFollow)) * b->ctx->numSMs;
     c.followChunks = c.numItems >= 4 * fResident ? 1 : follow_max_chunks_per_item(c.n);
     c.followBlocks = std::max(1, std::min(fResident, c.numItems * c.followChunks));
     return TFX_OK;
@@ -347,7 +343,7 @@ static int launch_strands(tfx_batch b, BatchClass& c, cudaStream_t s, bool after
 
 static int launch_follows(tfx_batch b, BatchClass& c, cudaStream_t s) {
     if (!c.followWork) return TFX_OK;
-    FollowLaunch fl{c.n, c.followBlocks, b->objTable, c.items, c.numItems, c.followChunks, c.followMode,
+    FollowLaunch fl{c.n, c.followBlocks, b->objTable, c.items, c.numItems, c.followChunks,
                     c.noFollow ? 1 : 0};
     cudaError_t e = launch_follow_collide(fl, s);
     return e == cudaSuccess ? TFX_OK : cuda_fail(e, "tfx_batch: follow/collide launch");
@@ -626,17 +622,6 @@ static int autotune(tfx_batch b, int frames) {
             if (ms < best) { best = ms; bestCap = cap; }
         }
         c.vpl = bestV; c.warps = bestW; c.perSMCap = bestCap; c.splitSweeps = bestSplit;
-        // the follow/collide form: one vertex at a time, both lookup stages queued, or the gradient stage
-        int bestMode = c.followMode;
-        for (int mode = 0; rc == TFX_OK && mode < 3; ++mode) {
-            if (mode == bestMode) continue;
-            c.followMode = mode;
-            if ((rc = size_class(b, c))) break;
-            float ms;
-            if ((rc = time_graph_frames(b, frames, &ms))) break;
-            if (ms < 0.99f * best) { best = ms; bestMode = mode; }   // a measured default yields to a clear gain only
-        }
-        c.followMode = bestMode;
         if (rc == TFX_OK) rc = size_class(b, c);
     }
     int rr = snapshot_restore(sn, s);
@@ -1132,10 +1117,7 @@ extern "C" int tfx_batch_set_option(tfx_batch b, int option, int value) {
             break;
         case TFX_BATCH_FOLLOW_FORM:
             if (value < 0 || value > 2) return fail(TFX_ERR_INVALID_ARGUMENT, "tfx_batch_set_option: follow form %d", value);
-            for (auto& c : b->classes) {
-                c.followMode = value;
-                if (int r = size_class(b, c)) return r;
-            }
+            for (auto& c : b->classes) c.followForm = value;
             break;
         case TFX_BATCH_WAIT_POLLS:
             if (value < 0) return fail(TFX_ERR_INVALID_ARGUMENT, "tfx_batch_set_option: wait polls %d", value);
@@ -1164,7 +1146,7 @@ extern "C" int tfx_batch_get_option(tfx_batch b, int option, int* value) {
         case TFX_BATCH_OVERLAP_SDF: *value = b->overlap ? 1 : 0; break;
         case TFX_BATCH_SDF_BLOCK: *value = b->sdfL.constructThreads; break;
         case TFX_BATCH_SPLIT_SWEEPS: *value = (!b->classes.empty() && b->classes[0].splitSweeps) ? 1 : 0; break;
-        case TFX_BATCH_FOLLOW_FORM: *value = b->classes.empty() ? 0 : b->classes[0].followMode; break;
+        case TFX_BATCH_FOLLOW_FORM: *value = b->classes.empty() ? 0 : b->classes[0].followForm; break;
         case TFX_BATCH_WAIT_POLLS: *value = b->waitPolls; break;
         case TFX_BATCH_SDF_FORM: *value = b->sdfForm; break;
         default: return fail(TFX_ERR_INVALID_ARGUMENT, "tfx_batch_get_option: unknown option %d", option);

@@ -757,117 +757,49 @@ __global__ void __launch_bounds__(128) k_local_sweep(const BatchObject* __restri
     }
 }
 
-// GetSignedDistance + TrilinearInterpolate (TressFXSDFCollision.hlsl:414-527) on the corner-expanded
-// grid: the same cell, bounds test, corner values and interpolation as sdf_lookup.
-__device__ __forceinline__ float sdf_lookup8(const float4* __restrict__ sdf8, const SdfGrid& g, float3 p) {
-    if (sdf_surely_outside(g, p)) return 1e10f;
-    const int3 gc = sdf_coords(g, p);
-    if (!(0 <= gc.x && gc.x < g.nx - 2) || !(0 <= gc.y && gc.y < g.ny - 2) || !(0 <= gc.z && gc.z < g.nz - 2))
-        return 1e10f;
-    const long long base = ((long long)g.ny * g.nx) * gc.z + (long long)g.nx * gc.y + gc.x;
-    const float4 lo = __ldg(sdf8 + 2 * base), hi = __ldg(sdf8 + 2 * base + 1);
-    const float d[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-        if (d[j] == 1e10f) return 1e10f;
-    const float3 cp = sdf_cell_pos(g, gc.x, gc.y, gc.z);
-    const float3 ip = divs(sub(p, cp), g.cell);
-    const float b0 = lerp_ref(lerp_ref(d[0], d[1], ip.x), lerp_ref(d[2], d[3], ip.x), ip.y);
-    const float b1 = lerp_ref(lerp_ref(d[4], d[5], ip.x), lerp_ref(d[6], d[7], ip.x), ip.y);
-    return lerp_ref(b0, b1, ip.z);
-}
-
-// sdf_collide_from with every lookup on the expanded grid.
-__device__ __forceinline__ bool sdf_collide_from8(const float4* __restrict__ sdf8, const SdfGrid& g, float margin,
-                                                  float3 p, float distance, float3& proj) {
-    if (distance > margin) return false;
-    const float h = 0.1f * g.cell;
-    const float fx = sdf_lookup8(sdf8, g, add(p, mul(mk3(1.0f, 0.0f, 0.0f), h)));
-    const float fy = sdf_lookup8(sdf8, g, add(p, mul(mk3(0.0f, 1.0f, 0.0f), h)));
-    const float fz = sdf_lookup8(sdf8, g, add(p, mul(mk3(0.0f, 0.0f, 1.0f), h)));
-    const float3 grad = mk3((fx - distance) / h, (fy - distance) / h, (fz - distance) / h);
-    const float3 nrm = normalize(grad);
-    if (distance < margin) {
-        proj = add(p, mul(nrm, margin - distance));
-        return true;
-    }
-    return false;
-}
-
-// The part of the collision after the first lookup (the vertices within the margin).
-__device__ __forceinline__ bool collide_near(const float* __restrict__ sdf, const float4* __restrict__ sdf8,
-                                             const SdfGrid& g, float margin, float3 p, float distance, float3* proj) {
-    float3 q = p;
-    const bool hit = sdf8 ? sdf_collide_from8(sdf8, g, margin, p, distance, q) : sdf_collide_from(sdf, g, margin, p, distance, q);
-    *proj = q;
-    return hit;
-}
-
-// What the vertices of one group share: the object's buffers, SDF, grid, margin, tip separation.
+// What the collided vertices of one group share: the SDF, its grid and margin.
 struct FollowGroup {
-    HairView h;
     const float* sdf;
     const float4* sdf8;
     SdfGrid sg;
-    float margin, tip;
-    int firstStrand;     // first strand of the group (guide strands and their follows)
+    SdfSteps st;
+    float margin;
 };
 
-__device__ __forceinline__ bool follow_group(const BatchObject& ob, const WorkItem& wi, FollowGroup& fg) {
-    fg.h = ob.hair;
+__device__ __forceinline__ bool follow_group(const BatchObject& ob, FollowGroup& fg) {
     fg.sdf = ob.sdf;
+    if (!fg.sdf) return false;
     fg.sdf8 = ob.sdf8;
-    if (fg.h.F == 0 && !fg.sdf) return false;
-    fg.sg = SdfGrid{0.f, 0.f, 0.f, 1.f, 0, 0, 0, 0};
-    fg.margin = 0.0f;
-    if (fg.sdf) { fg.sg = ob.sdfFrame->grid; fg.margin = ob.sdfFrame->margin; }
-    fg.tip = ob.consts->tipSeparation;
-    fg.firstStrand = wi.firstGuide * (fg.h.F + 1);
+    fg.sg = ob.sdfFrame->grid;
+    fg.margin = ob.sdfFrame->margin;
+    fg.st = sdf_steps(fg.sg, fg.margin);
     return true;
 }
 
-// Guide vertex e of a group: its follow vertices and the collision of all of them.  NF: every object
-// of the class has no follow hairs (F = 0 known at compile time, which frees registers).
-template <int N, bool NF>
-__device__ __forceinline__ void follow_collide_vertex(const FollowGroup& fg, int e) {
-    constexpr float kInvN = 1.0f / (float)N;   // exact: N is a power of two, so j * kInvN == j / N
-    const HairView& h = fg.h;
-    const int F = NF ? 0 : h.F;
-    const float* __restrict__ sdf = fg.sdf;
-    const float4* __restrict__ sdf8 = fg.sdf8;
-    const SdfGrid& sg = fg.sg;
-    const float margin = fg.margin, tip = fg.tip;
-    const int s = e / N, j = e % N;
-    const int gs = fg.firstStrand + s * (F + 1);
-    const size_t vg = (size_t)gs * N + j;
-    const float4 gp = h.pos[vg];
-    const float4 tn = F > 0 ? h.tan[vg] : make_float4(0.f, 0.f, 0.f, 0.f);   // copied to the follow vertices only
-    const bool collide = sdf && j >= 2;
-    const float factor = tip * ((float)j * kInvN) + 1.0f;
-    for (int i = 0; i <= F; ++i) {
-        const size_t v = vg + (size_t)i * N;
-        float3 pt = xyz(gp);
-        float w = gp.w;
-        if (i > 0) {
-            const float4 off = __ldg(h.followOffset + gs + i);
-            pt = add(xyz(gp), mul(factor, xyz(off)));
-            // inverse mass of the follow vertex: only this thread writes the word, after this read
-            w = __ldg(&h.pos[v].w);
-        }
-        float3 proj = pt;
-        bool hit = false;
-        if (collide) {
-            const float dist = sdf8 ? sdf_lookup8(sdf8, sg, pt) : sdf_lookup(sdf, sg, pt);
-            if (dist <= margin) hit = collide_near(sdf, sdf8, sg, margin, pt, dist, &proj);
-        }
-        if (i > 0) {
-            h.pos[v] = make_float4(proj.x, proj.y, proj.z, w);
-            h.tan[v] = tn;
-        } else if (hit) {
-            h.pos[v] = with_xyz(gp, proj);
-        }
-        if (hit) h.prev[v] = with_xyz(h.prev[v], proj);
+// A cell's corners from the corner-expanded copy where there is one.
+struct GroupCorners {
+    GridCorners grid;
+    const float4* sdf8;
+    __device__ __forceinline__ void corners(int base, float (&d)[8]) const {
+        if (!sdf8) return grid.corners(base, d);
+        const float4* r = sdf8 + 2 * (long long)base;
+        const float4 lo = __ldg(r), hi = __ldg(r + 1);
+        d[0] = lo.x; d[1] = lo.y; d[2] = lo.z; d[3] = lo.w;
+        d[4] = hi.x; d[5] = hi.y; d[6] = hi.z; d[7] = hi.w;
     }
+    // straight from the grid: a tenth of the lanes read these, and reading them from the records measured slower
+    __device__ __forceinline__ float4 beyond_x(int base) const { return grid.beyond_x(base); }
+    __device__ __forceinline__ float4 beyond_y(int base) const { return grid.beyond_y(base); }
+    __device__ __forceinline__ float4 beyond_z(int base) const { return grid.beyond_z(base); }
+};
+
+// The collision of a vertex at p against the group's SDF.
+__device__ __forceinline__ bool follow_collide_point(const FollowGroup& fg, float3 p, float3& proj) {
+    return sdf_collide_cell(fg.sdf, fg.sg, fg.st, fg.margin, p, proj, GroupCorners{GridCorners(fg.sdf, fg.sg), fg.sdf8});
+}
+__device__ __forceinline__ void store_xyz(float4* p, float3 v) {
+    *reinterpret_cast<float2*>(p) = make_float2(v.x, v.y);
+    p->z = v.z;
 }
 
 // ============================================================================================
@@ -875,175 +807,68 @@ __device__ __forceinline__ void follow_collide_vertex(const FollowGroup& fg, int
 //
 // UpdateFollowHairVertices (TressFXSimulation.hlsl:978-1001) and CollideHairVerticesWithSdf_forward
 // (TressFXSDFCollision.hlsl:531-595) for the groups of one vertices-per-strand class, after
-// k_fused_strands has written the guides' constrained state and the frame's SDFs are built.  One
-// thread per guide vertex; it makes the vertex's F follow vertices (hair i = 1..F) from the guide's
-// pre-collision position, then collides the guide vertex and every follow vertex (one vertex at a
-// time: at 64 registers four blocks fit per SM, and that occupancy hides the gathers better than
-// loads of several hairs in flight per thread did).  Each group
-// is cut into chunksPerItem chunks of guide vertices (a multiple of 256), which persistent blocks take
-// in turn: with few groups per block, smaller chunks spread groups of unequal cost (collisions) evenly
-// over the SMs; with many, whole groups keep the per-chunk overhead low.
-template <int N, bool NF>
-__global__ void __launch_bounds__(256, NF ? 5 : 4) k_follow_collide(const BatchObject* __restrict__ objs,
-                                                           const WorkItem* __restrict__ items, int numItems,
-                                                           int chunksPerItem) {
-    constexpr int kGroupVerts = fused_group_strands(N) * N;
-    const int chunkLen = ((kGroupVerts + chunksPerItem - 1) / chunksPerItem + 255) & ~255;
-    const int numChunks = numItems * chunksPerItem;
-    for (int c = blockIdx.x; c < numChunks; c += gridDim.x) {
-        const int it = c / chunksPerItem;
-        const WorkItem wi = items[it];
-        const int begin = (c - it * chunksPerItem) * chunkLen;
-        const int end = min(begin + chunkLen, wi.count * N);
-        FollowGroup fg;
-        if (!follow_group(objs[wi.obj], wi, fg)) continue;
-        for (int e = begin + (int)threadIdx.x; e < end; e += blockDim.x) follow_collide_vertex<N, NF>(fg, e);
-    }
-}
-
-// ============================================================================================
-// follow hairs + collision with per-warp lookup queues (classes whose objects have follow hairs)
+// k_fused_strands has written the guides' constrained state and the frame's SDFs are built.  Each group
+// is cut into chunksPerItem chunks of whole guide strands (a multiple of the block's threads in guide
+// vertices), which persistent blocks take in turn: with few groups per block, smaller chunks spread groups
+// of unequal cost (collisions) evenly over the SMs; with many, whole groups keep the per-chunk
+// overhead low.  A block first makes its chunk's follow vertices from the guides, a thread per guide
+// vertex, then collides all the chunk's vertices, which lie one after the other in memory, a thread
+// per vertex.  NF: no object of the class has follow hairs.
 //
-// The same work as k_follow_collide, with the warp's lanes decoupled from its lookups: lane l owns one
-// guide vertex, makes and writes its follow vertices, and queues every vertex (guide or follow) the
-// collision may move (j >= 2, not certainly outside the grid).  The warp runs the first lookup on 32
-// queued vertices at a time, then the gradient stage on 32 of those within the margin at a time, so
-// both run on full warps: a strand reaches from the scalp, where vertices touch the surface, out to
-// tips far from it, and with follow hairs a lane has F + 1 vertices of that mix.  A moved vertex gets
-// Pos and Prev from the lane that collided it, after the owner's write of the follow's Pos
-// (__syncwarp orders the two).  The queues are emptied at the end of each chunk.
-constexpr int kFollowWarps = 8;
-struct FollowQueues {
-    int idx1[kFollowWarps][64];      // stage 1: offset of the vertex in the group
-    float4 pos1[kFollowWarps][64];   //          its position and inverse mass
-    int idx2[kFollowWarps][64];      // stage 2: the same, for vertices within the margin
-    float4 pos2[kFollowWarps][64];
-    float dist2[kFollowWarps][64];   //          and their first lookup's distance
-};
-
-// Lane k < n takes entry k of a queue; the entries from 32 on move to the front.
-__device__ __forceinline__ bool queue_take(int* idx, float4* pos, float* dist, int& n, int lane, int& ri, float4& rp,
-                                           float& rd) {
-    __syncwarp();
-    const bool have = lane < n;
-    if (have) { ri = idx[lane]; rp = pos[lane]; if (dist) rd = dist[lane]; }
-    __syncwarp();
-    if (lane < n - 32) { idx[lane] = idx[lane + 32]; pos[lane] = pos[lane + 32]; if (dist) dist[lane] = dist[lane + 32]; }
-    __syncwarp();
-    n = max(n - 32, 0);
-    return have;
-}
-
-// Stage 2 on up to 32 queued vertices: the gradient lookups and, inside the margin, the projection.
-__device__ __forceinline__ void follow_stage2(const FollowGroup& fg, size_t vbase, FollowQueues& Q, int warp, int lane,
-                                              int& n2) {
-    int ri = 0; float4 rp = make_float4(0.f, 0.f, 0.f, 0.f); float rd = 0.0f;
-    if (!queue_take(Q.idx2[warp], Q.pos2[warp], Q.dist2[warp], n2, lane, ri, rp, rd)) return;
-    float3 proj;
-    if (collide_near(fg.sdf, fg.sdf8, fg.sg, fg.margin, xyz(rp), rd, &proj)) {
-        const size_t v = vbase + (size_t)ri;
-        fg.h.pos[v] = make_float4(proj.x, proj.y, proj.z, rp.w);
-        fg.h.prev[v] = with_xyz(fg.h.prev[v], proj);
-    }
-}
-
-// Stage 1 on up to 32 queued vertices: the first lookup; those within the margin join stage 2.
-__device__ __forceinline__ void follow_stage1(const FollowGroup& fg, size_t vbase, FollowQueues& Q, int warp, int lane,
-                                              int& n1, int& n2) {
-    int ri = 0; float4 rp = make_float4(0.f, 0.f, 0.f, 0.f); float rd = 0.0f;
-    const bool have = queue_take(Q.idx1[warp], Q.pos1[warp], nullptr, n1, lane, ri, rp, rd);
-    bool near = false;
-    if (have) {
-        rd = fg.sdf8 ? sdf_lookup8(fg.sdf8, fg.sg, xyz(rp)) : sdf_lookup(fg.sdf, fg.sg, xyz(rp));
-        near = rd <= fg.margin;
-    }
-    const unsigned m = __ballot_sync(0xffffffffu, near);
-    if (near) {
-        const int k = n2 + __popc(m & ((1u << lane) - 1u));
-        Q.idx2[warp][k] = ri; Q.pos2[warp][k] = rp; Q.dist2[warp][k] = rd;
-    }
-    n2 += __popc(m);
-    if (n2 >= 32) follow_stage2(fg, vbase, Q, warp, lane, n2);
-}
-
-// QueueFirst = false: each lane runs its vertices' first lookup itself and only the vertices within
-// the margin are queued (for classes without follow hairs, where a lane has one vertex per step).
-template <int N, bool QueueFirst, bool NF>
-__global__ void __launch_bounds__(256, NF ? 5 : 4) k_follow_collide_queued(const BatchObject* __restrict__ objs,
-                                                                  const WorkItem* __restrict__ items, int numItems,
-                                                                  int chunksPerItem) {
+// Bound by the gathers of the collision (without the corner-expanded copy the head's frame takes 133 us
+// in place of 108) and by how many warps hide them: 64 registers and eight blocks of 128 an SM, at which
+// next to nothing spills once making the follow vertices is a loop of its own.  A thread that made and
+// collided its guide's F + 1 vertices in turn took 80 registers and 112 us a frame of the head, 43.2 of
+// the character (spilling to 64: 124 and 41.0); this form 108.5 and 40.7.  Before the shared corners
+// (sdf_collide_cell), with per-warp queues of the vertices within the margin: 117 and 41.0; 200,000
+// strands of 16 without follow hairs 283 us, now 259.
+constexpr int kFollowThreads = 128, kFollowBlocksPerSM = 8;
+template <int N, bool NF>
+__global__ void __launch_bounds__(kFollowThreads, kFollowBlocksPerSM) k_follow_collide(const BatchObject* __restrict__ objs,
+                                                                      const WorkItem* __restrict__ items, int numItems,
+                                                                      int chunksPerItem) {
     constexpr int kGroupVerts = fused_group_strands(N) * N;
     constexpr float kInvN = 1.0f / (float)N;   // exact: N is a power of two, so j * kInvN == j / N
-    __shared__ FollowQueues Q;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const unsigned below = (1u << lane) - 1u;
-    const int chunkLen = ((kGroupVerts + chunksPerItem - 1) / chunksPerItem + 255) & ~255;
+    const int chunkLen = ((kGroupVerts + chunksPerItem - 1) / chunksPerItem + kFollowThreads - 1) & ~(kFollowThreads - 1);
     const int numChunks = numItems * chunksPerItem;
     for (int c = blockIdx.x; c < numChunks; c += gridDim.x) {
         const int it = c / chunksPerItem;
         const WorkItem wi = items[it];
         const int begin = (c - it * chunksPerItem) * chunkLen;
         const int end = min(begin + chunkLen, wi.count * N);
-        FollowGroup fg;
-        if (!follow_group(objs[wi.obj], wi, fg)) continue;
-        const HairView& h = fg.h;
-        const int F = NF ? 0 : h.F;
-        const size_t vbase = (size_t)fg.firstStrand * N;
-        int n1 = 0, n2 = 0;
-        for (int base = begin + warp * 32; base < end; base += blockDim.x) {
-            const int e = base + lane;
-            const bool active = e < end;
-            const int s = e / N, j = e % N;
-            const int gs = fg.firstStrand + s * (F + 1);
-            const size_t vg = (size_t)gs * N + j;
-            float4 gp = make_float4(0.f, 0.f, 0.f, 0.f), tn = gp;
-            if (active) {
-                gp = h.pos[vg];
-                if (F > 0) tn = h.tan[vg];   // copied to the follow vertices only
+        if (begin >= end) continue;
+        const BatchObject& ob = objs[wi.obj];
+        const int F1 = NF ? 1 : ob.hair.F + 1;
+        if (!NF && F1 > 1) {
+            const HairView h = ob.hair;
+            const float tip = ob.consts->tipSeparation;
+            for (int e = begin + (int)threadIdx.x; e < end; e += kFollowThreads) {
+                const int gs = (wi.firstGuide + e / N) * F1, j = e % N;
+                const size_t vg = (size_t)gs * N + j;
+                const float3 gp = xyz(h.pos[vg]);
+                const float4 tn = h.tan[vg];
+                const float factor = tip * ((float)j * kInvN) + 1.0f;
+#pragma unroll 4
+                for (int i = 1; i < F1; ++i) {
+                    const float3 pt = add(gp, mul(factor, xyz(__ldg(h.followOffset + gs + i))));
+                    store_xyz(h.pos + vg + (size_t)i * N, pt);   // w, the inverse mass, stays
+                    h.tan[vg + (size_t)i * N] = tn;
+                }
             }
-            const bool collide = active && fg.sdf && j >= 2;
-            const float factor = fg.tip * ((float)j * kInvN) + 1.0f;
-            for (int i = 0; i <= F; ++i) {
-                const size_t v = vg + (size_t)i * N;
-                float3 pt = xyz(gp);
-                float w = gp.w;
-                if (active && i > 0) {
-                    const float4 off = __ldg(h.followOffset + gs + i);
-                    pt = add(xyz(gp), mul(factor, xyz(off)));
-                    // inverse mass of the follow vertex: only this lane writes the word, after this read
-                    w = __ldg(&h.pos[v].w);
-                    h.pos[v] = make_float4(pt.x, pt.y, pt.z, w);
-                    h.tan[v] = tn;
-                }
-                const bool need = collide && !sdf_surely_outside(fg.sg, pt);
-                if (QueueFirst) {
-                    const unsigned m = __ballot_sync(0xffffffffu, need);
-                    if (need) {
-                        const int k = n1 + __popc(m & below);
-                        Q.idx1[warp][k] = (int)(v - vbase);
-                        Q.pos1[warp][k] = make_float4(pt.x, pt.y, pt.z, w);
-                    }
-                    n1 += __popc(m);
-                    if (n1 >= 32) follow_stage1(fg, vbase, Q, warp, lane, n1, n2);
-                } else {
-                    float d = 0.0f;
-                    if (need) d = fg.sdf8 ? sdf_lookup8(fg.sdf8, fg.sg, pt) : sdf_lookup(fg.sdf, fg.sg, pt);
-                    const bool near = need && d <= fg.margin;
-                    const unsigned m = __ballot_sync(0xffffffffu, near);
-                    if (near) {
-                        const int k = n2 + __popc(m & below);
-                        Q.idx2[warp][k] = (int)(v - vbase);
-                        Q.pos2[warp][k] = make_float4(pt.x, pt.y, pt.z, w);
-                        Q.dist2[warp][k] = d;
-                    }
-                    n2 += __popc(m);
-                    if (n2 >= 32) follow_stage2(fg, vbase, Q, warp, lane, n2);
-                }
+            __syncthreads();
+        }
+        FollowGroup fg;
+        if (!follow_group(ob, fg)) continue;
+        float4* pos = ob.hair.pos + ((size_t)wi.firstGuide * N + begin) * F1;
+        float4* prev = ob.hair.prev + ((size_t)wi.firstGuide * N + begin) * F1;
+        for (int e = threadIdx.x; e < (end - begin) * F1; e += kFollowThreads) {
+            if (e % N < 2) continue;
+            float3 proj;
+            if (follow_collide_point(fg, xyz(pos[e]), proj)) {
+                store_xyz(pos + e, proj);
+                store_xyz(prev + e, proj);   // w stays: no load for the store to wait for
             }
         }
-        while (n1 > 0) follow_stage1(fg, vbase, Q, warp, lane, n1, n2);
-        while (n2 > 0) follow_stage2(fg, vbase, Q, warp, lane, n2);
-        __syncwarp();
     }
 }
 
@@ -1168,16 +993,11 @@ int fused_blocks_per_sm(int n, int vpl, int warps) {
     return 0;
 }
 
-int follow_max_chunks_per_item(int n) { return (fused_group_strands(n) * n + 255) / 256; }
+int follow_max_chunks_per_item(int n) { return (fused_group_strands(n) * n + kFollowThreads - 1) / kFollowThreads; }
 
 template <int N, bool NF>
 static cudaError_t launch_follow_nf(const FollowLaunch& fl, cudaStream_t s) {
-    if (fl.queued == 1)
-        k_follow_collide_queued<N, true, NF><<<fl.blocks, 256, 0, s>>>(fl.objs, fl.items, fl.numItems, fl.chunks);
-    else if (fl.queued == 2)
-        k_follow_collide_queued<N, false, NF><<<fl.blocks, 256, 0, s>>>(fl.objs, fl.items, fl.numItems, fl.chunks);
-    else
-        k_follow_collide<N, NF><<<fl.blocks, 256, 0, s>>>(fl.objs, fl.items, fl.numItems, fl.chunks);
+    k_follow_collide<N, NF><<<fl.blocks, kFollowThreads, 0, s>>>(fl.objs, fl.items, fl.numItems, fl.chunks);
     return cudaGetLastError();
 }
 
@@ -1187,12 +1007,9 @@ static cudaError_t launch_follow_n(const FollowLaunch& fl, cudaStream_t s) {
 }
 
 template <bool NF>
-static cudaError_t follow_occupancy(int n, int mode, int* nb) {
-#define TFX_FOLLOW_OCC(NN)                                                                                                \
-    case NN:                                                                                                              \
-        return mode == 1   ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(nb, k_follow_collide_queued<NN, true, NF>, 256, 0)  \
-               : mode == 2 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(nb, k_follow_collide_queued<NN, false, NF>, 256, 0) \
-                           : cudaOccupancyMaxActiveBlocksPerMultiprocessor(nb, k_follow_collide<NN, NF>, 256, 0);
+static cudaError_t follow_occupancy(int n, int* nb) {
+#define TFX_FOLLOW_OCC(NN) \
+    case NN: return cudaOccupancyMaxActiveBlocksPerMultiprocessor(nb, k_follow_collide<NN, NF>, kFollowThreads, 0);
     switch (n) {
         TFX_FOLLOW_OCC(4)
         TFX_FOLLOW_OCC(8)
@@ -1204,9 +1021,9 @@ static cudaError_t follow_occupancy(int n, int mode, int* nb) {
 #undef TFX_FOLLOW_OCC
 }
 
-int follow_blocks_per_sm(int n, int mode, bool noFollow) {
+int follow_blocks_per_sm(int n, bool noFollow) {
     int nb = 0;
-    const cudaError_t e = noFollow ? follow_occupancy<true>(n, mode, &nb) : follow_occupancy<false>(n, mode, &nb);
+    const cudaError_t e = noFollow ? follow_occupancy<true>(n, &nb) : follow_occupancy<false>(n, &nb);
     return e == cudaSuccess ? nb : 0;
 }
 

@@ -88,20 +88,11 @@ __global__ void __launch_bounds__(256) k_sdf_collide(const float* __restrict__ s
     after_previous();
     const long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (v >= vtot) return;
-    const int local = (int)(v % n);
+    const int local = v >> 32 ? (int)(v % n) : (int)((uint32_t)v % (uint32_t)n);
     if (local == 0 || local == 1) return;
     const float4 hv = pos[v];
-    const float3 p = xyz(hv);
-    const float distance = sdf_lookup(sdf, g, p);
-    if (distance > margin) return;
-    const float h = 0.1f * g.cell;
-    const float fx = sdf_lookup(sdf, g, add(p, mul(mk3(1.0f, 0.0f, 0.0f), h)));
-    const float fy = sdf_lookup(sdf, g, add(p, mul(mk3(0.0f, 1.0f, 0.0f), h)));
-    const float fz = sdf_lookup(sdf, g, add(p, mul(mk3(0.0f, 0.0f, 1.0f), h)));
-    const float3 grad = mk3((fx - distance) / h, (fy - distance) / h, (fz - distance) / h);
-    const float3 nrm = normalize(grad);
-    if (distance < margin) {
-        const float3 proj = add(p, mul(nrm, margin - distance));
+    float3 proj;
+    if (sdf_collide_point(sdf, g, margin, xyz(hv), proj)) {
         pos[v] = with_xyz(hv, proj);
         const float4 pv = prev[v];
         prev[v] = with_xyz(pv, proj);

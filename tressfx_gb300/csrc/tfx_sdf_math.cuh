@@ -483,25 +483,8 @@ __device__ __forceinline__ float sdf_lookup(const float* __restrict__ sdf, const
 
 // CollideHairVerticesWithSdf_forward for one vertex (j >= 2): returns true and the projected
 // position when the vertex is pushed out (then Pos.xyz and Prev.xyz both take it).
-// The part after the first lookup: `distance` = sdf_lookup(sdf, g, p).
-__device__ __forceinline__ bool sdf_collide_from(const float* __restrict__ sdf, const SdfGrid& g, float margin, float3 p,
-                                                 float distance, float3& proj) {
-    if (distance > margin) return false;
-    const float h = 0.1f * g.cell;
-    const float fx = sdf_lookup(sdf, g, add(p, mul(mk3(1.0f, 0.0f, 0.0f), h)));
-    const float fy = sdf_lookup(sdf, g, add(p, mul(mk3(0.0f, 1.0f, 0.0f), h)));
-    const float fz = sdf_lookup(sdf, g, add(p, mul(mk3(0.0f, 0.0f, 1.0f), h)));
-    const float3 grad = mk3((fx - distance) / h, (fy - distance) / h, (fz - distance) / h);
-    const float3 nrm = normalize(grad);
-    if (distance < margin) {
-        proj = add(p, mul(nrm, margin - distance));
-        return true;
-    }
-    return false;
-}
-
-__device__ __forceinline__ bool sdf_collide_point(const float* __restrict__ sdf, const SdfGrid& g, float margin, float3 p,
-                                                  float3& proj) {
+// In the shader's own form: the lookup at p and three more, 0.1 cells along each axis.
+static __device__ __noinline__ bool sdf_collide_general(const float* __restrict__ sdf, SdfGrid g, float margin, float3 p, float3* proj) {
     const float distance = sdf_lookup(sdf, g, p);
     if (distance > margin) return false;
     const float h = 0.1f * g.cell;
@@ -511,10 +494,134 @@ __device__ __forceinline__ bool sdf_collide_point(const float* __restrict__ sdf,
     const float3 grad = mk3((fx - distance) / h, (fy - distance) / h, (fz - distance) / h);
     const float3 nrm = normalize(grad);
     if (distance < margin) {
-        proj = add(p, mul(nrm, margin - distance));
+        *proj = add(p, mul(nrm, margin - distance));
         return true;
     }
     return false;
+}
+
+// The grid's two divisors, the cell size and the gradient's step, with their reciprocals for the short
+// exact division, made once per thread; `ranged` is false where the short form's ranges do not hold.
+struct SdfSteps {
+    float rcell, h, rh;
+    bool ranged;
+};
+__device__ __forceinline__ SdfSteps sdf_steps(const SdfGrid& g, float margin) {
+    SdfSteps s;
+    s.h = 0.1f * g.cell;
+    s.rcell = 1.0f / g.cell;
+    s.rh = 1.0f / s.h;
+    s.ranged = g.cell >= 16.0f * kDivisorMin && g.cell <= kDivisorMax && fabsf(g.ox) <= 0x1p90f && fabsf(g.oy) <= 0x1p90f &&
+               fabsf(g.oz) <= 0x1p90f && margin < 1e10f && (long long)g.nx * g.ny * g.nz < (1ll << 31);
+    return s;
+}
+// At least kDivKey for the numerators div_by is exact for: zero, and magnitudes from kDivMin on.
+__device__ __forceinline__ uint32_t div_key(float a) { return (__float_as_uint(a) & 0x7fffffffu) - 1u; }
+constexpr uint32_t kDivKey = 0x21800000u - 1u;   // kDivMin's bits, less one
+__device__ __forceinline__ bool div_keys(float a, float b, float c) { return min(min(div_key(a), div_key(b)), div_key(c)) >= kDivKey; }
+
+// The same result from the corners of one cell.  Along each axis the probe lies in p's cell (nine of
+// ten) or in the next: its lookup shares the other two axes' fractions with p's, and takes p's corners or
+// their far half and four new ones.  So a vertex reads 8 corners and, for a probe that leaves the cell,
+// 4 more, in place of 32, does 7 + 4 + 2 interpolations for the gradient in place of 21, and 8 divisions, in
+// their short form, in place of 27.  corners(base, d) gives the 8 corners of the cell at index base.
+constexpr int kCollideMiss = 0, kCollideHit = 1, kCollideGeneral = 2;
+template <class Corners>
+__device__ __forceinline__ int sdf_collide_shared(const float* __restrict__ sdf, const SdfGrid& g, const SdfSteps& st, float margin,
+                                                 float3 p, float3& proj, const Corners& cell) {
+    if (!st.ranged) return kCollideGeneral;
+    if (sdf_surely_outside(g, p)) return kCollideMiss;
+    // a numerator below the short form's range gives a quotient below 1 by either form
+    auto coord = [&](float d) { return ftoi(div_by(d, g.cell, st.rcell)); };
+    const int x = coord(p.x - g.ox), y = coord(p.y - g.oy), z = coord(p.z - g.oz);
+    if (!(0 <= x && x < g.nx - 2) || !(0 <= y && y < g.ny - 2) || !(0 <= z && z < g.nz - 2)) return kCollideMiss;
+    const int Y = g.nx, Z = g.ny * g.nx;
+    const int base = Z * z + Y * y + x;
+    float d[8];
+    cell.corners(base, d);
+    bool far = false;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) far |= d[j] == 1e10f;
+    if (far) return kCollideMiss;
+    const float3 cp = sdf_cell_pos(g, x, y, z);
+    const float3 a = sub(p, cp);
+    const float3 ip = mk3(div_by(a.x, g.cell, st.rcell), div_by(a.y, g.cell, st.rcell), div_by(a.z, g.cell, st.rcell));
+    const float x00 = lerp_ref(d[0], d[1], ip.x), x10 = lerp_ref(d[2], d[3], ip.x);
+    const float x01 = lerp_ref(d[4], d[5], ip.x), x11 = lerp_ref(d[6], d[7], ip.x);
+    const float b0 = lerp_ref(x00, x10, ip.y), b1 = lerp_ref(x01, x11, ip.y);
+    const float distance = lerp_ref(b0, b1, ip.z);
+    if (!div_keys(a.x, a.y, a.z)) return kCollideGeneral;
+    if (!(distance < margin)) return kCollideMiss;
+
+    const float qx = p.x + st.h, qy = p.y + st.h, qz = p.z + st.h;
+    const int px = coord(qx - g.ox), py = coord(qy - g.oy), pz = coord(qz - g.oz);
+    const bool mx = px != x, my = py != y, mz = pz != z;
+    const bool ox = px >= g.nx - 2, oy = py >= g.ny - 2, oz = pz >= g.nz - 2;   // past the grid: the lookup's 1e10
+    float4 e = make_float4(0.f, 0.f, 0.f, 0.f), f = e, k = e;
+    if (mx && !ox) e = cell.beyond_x(base);
+    if (my && !oy) f = cell.beyond_y(base);
+    if (mz && !oz) k = cell.beyond_z(base);
+    const float ax = qx - ((float)px * g.cell + g.ox), ay = qy - ((float)py * g.cell + g.oy), az = qz - ((float)pz * g.cell + g.oz);
+    const float tx = div_by(ax, g.cell, st.rcell), ty = div_by(ay, g.cell, st.rcell), tz = div_by(az, g.cell, st.rcell);
+    float fx = lerp_ref(lerp_ref(lerp_ref(mx ? d[1] : d[0], mx ? e.x : d[1], tx), lerp_ref(mx ? d[3] : d[2], mx ? e.y : d[3], tx), ip.y),
+                        lerp_ref(lerp_ref(mx ? d[5] : d[4], mx ? e.z : d[5], tx), lerp_ref(mx ? d[7] : d[6], mx ? e.w : d[7], tx), ip.y),
+                        ip.z);
+    if (ox || e.x == 1e10f || e.y == 1e10f || e.z == 1e10f || e.w == 1e10f) fx = 1e10f;
+    float fy = lerp_ref(lerp_ref(my ? x10 : x00, my ? lerp_ref(f.x, f.y, ip.x) : x10, ty),
+                        lerp_ref(my ? x11 : x01, my ? lerp_ref(f.z, f.w, ip.x) : x11, ty), ip.z);
+    if (oy || f.x == 1e10f || f.y == 1e10f || f.z == 1e10f || f.w == 1e10f) fy = 1e10f;
+    float fz = lerp_ref(mz ? b1 : b0, mz ? lerp_ref(lerp_ref(k.x, k.y, ip.x), lerp_ref(k.z, k.w, ip.x), ip.y) : b1, tz);
+    if (oz || k.x == 1e10f || k.y == 1e10f || k.z == 1e10f || k.w == 1e10f) fz = 1e10f;
+    const float gx = fx - distance, gy = fy - distance, gz = fz - distance;
+    // the shader adds 0 to the other two coordinates of a probe, which changes a zero's sign; a difference
+    // of zeros has a sign too; a step that spans more than a cell (a cell near p's rounding) shares nothing
+    const bool shared = (unsigned)(px - x) <= 1u && (unsigned)(py - y) <= 1u && (unsigned)(pz - z) <= 1u && p.x != 0.0f &&
+                        p.y != 0.0f && p.z != 0.0f && distance != 0.0f && div_keys(ax, ay, az) && div_keys(gx, gy, gz) &&
+                        fmaxf(fmaxf(fabsf(gx), fabsf(gy)), fabsf(gz)) <= 0x1p100f;
+    if (!shared) return kCollideGeneral;
+    const float3 nrm = normalize(mk3(div_by(gx, st.h, st.rh), div_by(gy, st.h, st.rh), div_by(gz, st.h, st.rh)));
+    proj = add(p, mul(nrm, margin - distance));
+    return kCollideHit;
+}
+
+template <class Corners>
+__device__ __forceinline__ bool sdf_collide_cell(const float* __restrict__ sdf, const SdfGrid& g, const SdfSteps& st, float margin,
+                                                 float3 p, float3& proj, const Corners& cell) {
+    const int r = sdf_collide_shared(sdf, g, st, margin, p, proj, cell);
+    if (r != kCollideGeneral) return r == kCollideHit;
+    float3 q;
+    if (!sdf_collide_general(sdf, g, margin, p, &q)) return false;
+    proj = q;
+    return true;
+}
+
+// The corners of cell `base` straight from the grid: its own 8, and the 4 that the next cell along an axis adds.
+struct GridCorners {
+    const float* sdf;
+    int Y, Z;
+    __device__ __forceinline__ GridCorners(const float* __restrict__ s, const SdfGrid& g) : sdf(s), Y(g.nx), Z(g.ny * g.nx) {}
+    __device__ __forceinline__ float4 four(const float* w, int a, int b, int c, int d) const {
+        return make_float4(__ldg(w + a), __ldg(w + b), __ldg(w + c), __ldg(w + d));
+    }
+    __device__ __forceinline__ void corners(int base, float (&d)[8]) const {
+        const float *w00 = sdf + base, *w10 = w00 + Y, *w01 = w00 + Z, *w11 = w01 + Y;
+        d[0] = __ldg(w00);
+        d[1] = __ldg(w00 + 1);
+        d[2] = __ldg(w10);
+        d[3] = __ldg(w10 + 1);
+        d[4] = __ldg(w01);
+        d[5] = __ldg(w01 + 1);
+        d[6] = __ldg(w11);
+        d[7] = __ldg(w11 + 1);
+    }
+    __device__ __forceinline__ float4 beyond_x(int base) const { return four(sdf + base + 2, 0, Y, Z, Z + Y); }
+    __device__ __forceinline__ float4 beyond_y(int base) const { return four(sdf + base + 2 * Y, 0, 1, Z, Z + 1); }
+    __device__ __forceinline__ float4 beyond_z(int base) const { return four(sdf + base + 2 * Z, 0, 1, Y, Y + 1); }
+};
+
+__device__ __forceinline__ bool sdf_collide_point(const float* __restrict__ sdf, const SdfGrid& g, float margin, float3 p,
+                                                  float3& proj) {
+    return sdf_collide_cell(sdf, g, sdf_steps(g, margin), margin, p, proj, GridCorners(sdf, g));
 }
 
 }  // namespace tfx
