@@ -93,9 +93,8 @@ struct SdfBatchLaunch {
     int totalTris;
     long long totalQuads;
     int constructThreads;
-    TriJob* jobs;         // [totalTris]: written by the initialisation, read by the construct; null when the
+    TriJob* jobs;         // [totalTris]: written before the construct reads it; null when the
                           // construct makes its own (sdf_takes_jobs)
-    bool after;      // the launch before it on the stream is a kernel it alone depends on (launch_after)
     int expand;      // some SDF keeps a corner-expanded copy: run the expansion
     // the SDFs that keep one, so that the expansion runs over their cells only: their indices into
     // `sdfs`, the prefix of their cell counts (nexp + 1 entries), and the sum
@@ -140,7 +139,10 @@ cudaError_t launch_follow_collide(const FollowLaunch& fl, cudaStream_t s);
 // CollideHairVerticesWithSdf_forward of one collision level's pairs
 cudaError_t launch_collide_level(const BatchObject* objs, const BatchSdf* sdfs, const BatchCollide* pairs, int npairs,
                                  long long totalVertices, cudaStream_t s);
-cudaError_t launch_batch_mesh_skin(const BatchMesh* meshes, int nmeshes, int totalVerts, cudaStream_t s);
+// Skins every mesh and gives every cell of the SDFs its initial word (totalQuads 0: no cell).
+cudaError_t launch_batch_mesh_skin(const BatchMesh* meshes, int nmeshes, int totalVerts, const BatchSdf* sdfs, int nsdf,
+                                   long long totalQuads, cudaStream_t s);
+cudaError_t prefer_strand_split();   // once per device before the first frame is captured
 cudaError_t launch_batch_sdf(const SdfBatchLaunch& l, cudaStream_t s);
 // Every object's positions, consecutively (first[i] = object i's first vertex), into `out` as float4 or packed xyz.
 cudaError_t launch_snapshot_positions(const BatchObject* objs, const long long* first, int nobj, long long total,

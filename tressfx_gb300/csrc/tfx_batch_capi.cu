@@ -308,12 +308,11 @@ static int size_class(tfx_batch b, BatchClass& c) {
 }
 
 static int launch_sdf_part(tfx_batch b, cudaStream_t s) {
-    if (b->totalMeshVerts > 0) {
-        cudaError_t e = launch_batch_mesh_skin(b->meshTable, b->nmeshes, b->totalMeshVerts, s);
-        if (e != cudaSuccess) return cuda_fail(e, "tfx_batch: mesh skinning launch");
-    }
+    // the tiled build sets its own words
+    cudaError_t e = launch_batch_mesh_skin(b->meshTable, b->nmeshes, b->totalMeshVerts, b->sdfTable, (int)b->sdfs.size(),
+                                           b->sdfForm == 1 || b->sdfs.empty() ? 0 : b->sdfL.totalQuads, s);
+    if (e != cudaSuccess) return cuda_fail(e, "tfx_batch: mesh skinning launch");
     if (!b->sdfs.empty()) {
-        cudaError_t e;
         if (b->sdfForm == 1) {
             e = launch_sdf_tiles(b->sdfT, s);
             if (e == cudaSuccess) e = launch_batch_sdf_expand(b->sdfL, s);
@@ -468,9 +467,9 @@ static int capture_graphs(tfx_batch b) {
     int sdfLaunches = 0;
     if (!b->sdfs.empty()) {
         if (b->sdfForm == 1) sdfLaunches = (b->sdfT.totalTris > 0 ? 5 : 1) + (b->sdfL.expand ? 1 : 0);
-        else sdfLaunches = (b->sdfL.totalTris > 0 ? 3 : 2) + (b->sdfL.expand ? 1 : 0);
+        else sdfLaunches = 1 + (b->sdfL.totalTris > 0 ? 1 : 0) + (b->sdfL.jobs ? 1 : 0) + (b->sdfL.expand ? 1 : 0);
     }
-    int launches = (b->totalMeshVerts > 0 ? 1 : 0) + sdfLaunches;
+    int launches = (b->totalMeshVerts > 0 || (!b->sdfs.empty() && b->sdfForm == 0) ? 1 : 0) + sdfLaunches;
     for (auto& c : b->classes) launches += c.numItems > 0 ? (c.splitSweeps ? 3 : 1) + (c.followWork ? 1 : 0) : 0;
     if (b->uploadKernel) ++launches;
     for (size_t k = 0; k < b->levelPairs.size(); ++k) launches += b->levelVertices[k] > 0 ? 1 : 0;
@@ -866,7 +865,8 @@ extern "C" int tfx_batch_build(tfx_batch b, int reserved) {
     if (sdf_takes_jobs(firstTri))
         TFX_CUDA(cudaMalloc(&b->jobArena, sdf_job_bytes() * (size_t)firstTri), "tfx_batch: triangle jobs");
     b->sdfL = SdfBatchLaunch{b->sdfTable, nsdf, firstTri, firstQuad, 128, reinterpret_cast<TriJob*>(b->jobArena),
-                             b->totalMeshVerts > 0, 0, nullptr, nullptr, 0, 0};
+                             0, nullptr, nullptr, 0, 0};
+    if (nsdf > 0) TFX_CUDA(prefer_strand_split(), "tfx_batch: shared-memory split of the SDF kernels");
     b->expandMode = 2;
     if (int r = apply_expand_mode(b)) return r;
 

@@ -3,7 +3,7 @@
 //
 //  * k_batch_mesh_skin    - BoneSkinning (TressFXBoneSkinning.hlsl:57-94) over every vertex of every
 //                           collision mesh.
-//  * k_batch_sdf_init / k_batch_sdf_construct / k_batch_sdf_finalize
+//  * k_batch_mesh_skin (its last blocks) / k_batch_sdf_jobs / k_batch_sdf_construct / k_batch_sdf_finalize
 //                         - InitializeSignedDistanceField / ConstructSignedDistanceField /
 //                           FinalizeSignedDistanceField (TressFXSDFCollision.hlsl:301-412) of every
 //                           SDF.  The construct runs one warp per triangle: the lanes share the
@@ -42,10 +42,52 @@
 namespace tfx {
 
 // ============================================================================================
-// collision-mesh skinning over all meshes
-__global__ void __launch_bounds__(256) k_batch_mesh_skin(const BatchMesh* __restrict__ meshes, int nmeshes,
-                                                         int totalVerts) {
+// The cells of every SDF in quads of four (the last quad of an SDF may be partial), kQuadRun quads of a
+// thread at a time, so that their loads are in flight together and one search finds their SDFs.
+constexpr int kQuadRun = 4;
+struct QuadRun {
+    uint32_t* words[kQuadRun];   // first cell of the quad
+    int cells[kQuadRun];         // 4, less at the end of an SDF, 0 past the last quad
+};
+__device__ __forceinline__ QuadRun quad_run(const BatchSdf* __restrict__ sdfs, int nsdf, long long totalQuads, long long first) {
+    QuadRun r;
+    int lo = 0, hi = nsdf - 1;
+    while (lo < hi) {   // last SDF with firstQuad <= first
+        const int mid = (lo + hi + 1) >> 1;
+        if (sdfs[mid].firstQuad <= first) lo = mid; else hi = mid - 1;
+    }
+#pragma unroll
+    for (int k = 0; k < kQuadRun; ++k) {
+        const long long q = first + k * 256;
+        r.cells[k] = 0;
+        if (q >= totalQuads) continue;
+        while (lo + 1 < nsdf && sdfs[lo + 1].firstQuad <= q) ++lo;
+        const long long c = 4 * (q - sdfs[lo].firstQuad);
+        r.words[k] = sdfs[lo].words + c;
+        r.cells[k] = (int)min(4ll, sdfs[lo].numCells - c);
+    }
+    return r;
+}
+inline unsigned quad_blocks(long long totalQuads) { return (unsigned)((totalQuads + 256 * kQuadRun - 1) / (256 * kQuadRun)); }
+
+// ============================================================================================
+// collision-mesh skinning over all meshes, and, in the blocks from skinBlocks on, the words' initial value
+// (InitializeSignedDistanceField, TressFXSDFCollision.hlsl:301-312), which needs no mesh
+__global__ void __launch_bounds__(256) k_batch_mesh_skin(const BatchMesh* __restrict__ meshes, int nmeshes, int totalVerts,
+                                                         int skinBlocks, const BatchSdf* __restrict__ sdfs, int nsdf,
+                                                         long long totalQuads) {
     after_previous();
+    if ((int)blockIdx.x >= skinBlocks) {
+        const uint32_t v = float_flip3(1e10f);
+        const QuadRun r = quad_run(sdfs, nsdf, totalQuads, (long long)(blockIdx.x - skinBlocks) * (256 * kQuadRun) + threadIdx.x);
+#pragma unroll
+        for (int k = 0; k < kQuadRun; ++k) {
+            if (r.cells[k] == 4) *reinterpret_cast<uint4*>(r.words[k]) = make_uint4(v, v, v, v);
+            else
+                for (int i = 0; i < r.cells[k]; ++i) r.words[k][i] = v;
+        }
+        return;
+    }
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= totalVerts) return;
     int lo = 0, hi = nmeshes - 1;
@@ -72,15 +114,6 @@ __device__ __forceinline__ int find_by_prefix_tri(const BatchSdf* __restrict__ s
     }
     return lo;
 }
-__device__ __forceinline__ int find_by_prefix_quad(const BatchSdf* __restrict__ sdfs, int nsdf, long long q) {
-    int lo = 0, hi = nsdf - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (sdfs[mid].firstQuad <= q) lo = mid; else hi = mid - 1;
-    }
-    return lo;
-}
-
 // The job of triangle t of the batch's triangle list (which spans the SDFs).
 __device__ __forceinline__ TriJob batch_job(const BatchSdf* __restrict__ sdfs, int nsdf, int t) {
     const BatchSdf& s = sdfs[find_by_prefix_tri(sdfs, nsdf, t)];
@@ -91,45 +124,34 @@ __device__ __forceinline__ TriJob batch_job(const BatchSdf* __restrict__ sdfs, i
     return tri_job(s.frame->grid, s.words, x0, x1, x2);
 }
 
-// InitializeSignedDistanceField, :301-312: every cell of every SDF, 4 cells per thread (the last
-// quad of an SDF may be partial), and with a job array the job of every triangle.
-__global__ void __launch_bounds__(256) k_batch_sdf_init(const BatchSdf* __restrict__ sdfs, int nsdf, long long totalQuads,
-                                                        TriJob* __restrict__ jobs, int totalTris) {
+// The job of every triangle, a thread per triangle; a block's jobs go out through shared memory, in whole lines:
+// 20 us for 234,000 triangles of sixteen meshes, where jobs and words in one launch, at the jobs' 78
+// registers a thread, took 47 (the words now ride with the skinning).
+__global__ void __launch_bounds__(kJobThreads) k_batch_sdf_jobs(const BatchSdf* __restrict__ sdfs, int nsdf, TriJob* __restrict__ jobs,
+                                                                int totalTris) {
     after_previous();
-    const uint32_t v = float_flip3(1e10f);
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < totalTris; t += stride)
-        jobs[t] = batch_job(sdfs, nsdf, (int)t);
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < totalQuads; q += stride) {
-        const BatchSdf& s = sdfs[find_by_prefix_quad(sdfs, nsdf, q)];
-        const long long c = 4 * (q - s.firstQuad);
-        const long long cells = s.numCells;
-        uint32_t* g = s.words;
-        if (c + 4 <= cells) {
-            *reinterpret_cast<uint4*>(g + c) = make_uint4(v, v, v, v);
-        } else {
-            for (long long i = c; i < cells; ++i) g[i] = v;
-        }
-    }
+    __shared__ JobStage stage;
+    const int first = blockIdx.x * kJobThreads, t = first + threadIdx.x;
+    if (t < totalTris) stage.put(threadIdx.x, batch_job(sdfs, nsdf, t));
+    stage.write(jobs + first, min(kJobThreads, totalTris - first));
 }
 
 // FinalizeSignedDistanceField, :400-412
 __global__ void __launch_bounds__(256) k_batch_sdf_finalize(const BatchSdf* __restrict__ sdfs, int nsdf,
                                                             long long totalQuads) {
     after_previous();
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < totalQuads; q += stride) {
-        const BatchSdf& s = sdfs[find_by_prefix_quad(sdfs, nsdf, q)];
-        const long long c = 4 * (q - s.firstQuad);
-        const long long cells = s.numCells;
-        uint32_t* g = s.words;
-        if (c + 4 <= cells) {
-            uint4 u = *reinterpret_cast<uint4*>(g + c);
-            *reinterpret_cast<uint4*>(g + c) = make_uint4(ifloat_flip3(u.x), ifloat_flip3(u.y), ifloat_flip3(u.z),
-                                                          ifloat_flip3(u.w));
-        } else {
-            for (long long i = c; i < cells; ++i) g[i] = ifloat_flip3(g[i]);
-        }
+    const QuadRun r = quad_run(sdfs, nsdf, totalQuads, (long long)blockIdx.x * (256 * kQuadRun) + threadIdx.x);
+    uint4 u[kQuadRun];
+#pragma unroll
+    for (int k = 0; k < kQuadRun; ++k)
+        if (r.cells[k] == 4) u[k] = *reinterpret_cast<const uint4*>(r.words[k]);
+#pragma unroll
+    for (int k = 0; k < kQuadRun; ++k) {
+        if (r.cells[k] == 4)
+            *reinterpret_cast<uint4*>(r.words[k]) =
+                make_uint4(ifloat_flip3(u[k].x), ifloat_flip3(u[k].y), ifloat_flip3(u[k].z), ifloat_flip3(u[k].w));
+        else
+            for (int i = 0; i < r.cells[k]; ++i) r.words[k][i] = ifloat_flip3(r.words[k][i]);
     }
 }
 
@@ -166,7 +188,7 @@ __global__ void __launch_bounds__(256) k_batch_sdf_expand(const BatchSdf* __rest
     }
 }
 
-// ConstructSignedDistanceField, :329-397, over the jobs k_batch_sdf_init made (every SDF's triangles in
+// ConstructSignedDistanceField, :329-397, over the jobs k_batch_sdf_jobs made (every SDF's triangles in
 // one list).  WARPS = warps per block.
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? kConstructBlocksPerSM : 1) k_batch_sdf_construct(const TriJob* __restrict__ jobs, int totalTris) {
@@ -1039,9 +1061,11 @@ cudaError_t launch_follow_collide(const FollowLaunch& fl, cudaStream_t s) {
     }
 }
 
-cudaError_t launch_batch_mesh_skin(const BatchMesh* meshes, int nmeshes, int totalVerts, cudaStream_t s) {
-    if (totalVerts <= 0) return cudaSuccess;
-    k_batch_mesh_skin<<<(totalVerts + 255) / 256, 256, 0, s>>>(meshes, nmeshes, totalVerts);
+cudaError_t launch_batch_mesh_skin(const BatchMesh* meshes, int nmeshes, int totalVerts, const BatchSdf* sdfs, int nsdf,
+                                   long long totalQuads, cudaStream_t s) {
+    const unsigned skinBlocks = (unsigned)((totalVerts + 255) / 256), initBlocks = quad_blocks(totalQuads);
+    if (skinBlocks + initBlocks == 0) return cudaSuccess;
+    k_batch_mesh_skin<<<skinBlocks + initBlocks, 256, 0, s>>>(meshes, nmeshes, totalVerts, (int)skinBlocks, sdfs, nsdf, totalQuads);
     return cudaGetLastError();
 }
 
@@ -1092,20 +1116,34 @@ static int sdf_construct_blocks_per_sm(int threads) {
     return e == cudaSuccess && nb > 0 ? nb : 1;
 }
 
+// The SDF chain runs beside the strand kernels, which want an SM's memory split for shared memory.  An SM
+// changes its split only when it is empty, so kernels of another preference do not run beside theirs: with
+// the chain's kernels asking for the same split (they gather nothing that L1 would keep), the character's
+// frame takes 40.2 us in place of 42.9 and three uneven objects' 26.7 in place of 28.2.  The follow kernel,
+// whose gathers live from L1, keeps the default (200,000 strands of 16: 249 us, 286 with this split).
+cudaError_t prefer_strand_split() {
+    cudaError_t e = cudaSuccess;
+    auto set = [&](auto* kernel) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    };
+    set(k_batch_mesh_skin);
+    set(k_batch_sdf_jobs);
+    set(k_batch_sdf_construct<2>);
+    set(k_batch_sdf_construct<4>);
+    set(k_batch_sdf_construct<8>);
+    set(k_batch_sdf_construct_chunks);
+    set(k_batch_sdf_finalize);
+    set(k_batch_sdf_expand);
+    return e;
+}
+
 cudaError_t launch_batch_sdf(const SdfBatchLaunch& L, cudaStream_t s) {
     if (L.nsdf <= 0) return cudaSuccess;
     const long long q = L.totalQuads;
-    const unsigned gq = (unsigned)std::min<long long>((q + 255) / 256, (long long)sm_count() * 32);
-    const long long initWork = std::max<long long>(q, L.jobs ? L.totalTris : 0);
-    const unsigned gi = (unsigned)std::min<long long>((initWork + 255) / 256, (long long)sm_count() * 32);
-    const int njobs = L.jobs ? L.totalTris : 0;
     cudaError_t e = cudaSuccess;
-    if (L.after) {
-        e = launch_after(k_batch_sdf_init, gi, 256, 0, s, L.sdfs, L.nsdf, q, L.jobs, njobs);
-    } else {
-        k_batch_sdf_init<<<gi, 256, 0, s>>>(L.sdfs, L.nsdf, q, L.jobs, njobs);
-        e = cudaGetLastError();
-    }
+    if (L.totalTris > 0 && L.jobs)
+        e = launch_after(k_batch_sdf_jobs, (unsigned)((L.totalTris + kJobThreads - 1) / kJobThreads), kJobThreads, 0, s, L.sdfs, L.nsdf,
+                         L.jobs, L.totalTris);
     if (e != cudaSuccess) return e;
     if (L.totalTris > 0 && L.jobs) {
         const int wpb = L.constructThreads / 32;
@@ -1120,7 +1158,7 @@ cudaError_t launch_batch_sdf(const SdfBatchLaunch& L, cudaStream_t s) {
         const unsigned blocks = (unsigned)std::min<long long>((chunks + 3) / 4, (long long)sm_count() * 64);
         e = launch_after(k_batch_sdf_construct_chunks, blocks, 128, sdf_construct_smem(4, per), s, L.sdfs, L.nsdf, L.totalTris, per);
     }
-    if (e == cudaSuccess) e = launch_after(k_batch_sdf_finalize, gq, 256, 0, s, L.sdfs, L.nsdf, q);
+    if (e == cudaSuccess) e = launch_after(k_batch_sdf_finalize, quad_blocks(q), 256, 0, s, L.sdfs, L.nsdf, q);
     if (e != cudaSuccess || !L.expand) return e;
     return launch_batch_sdf_expand(L, s);
 }

@@ -427,6 +427,24 @@ struct SdfJobOrder {
     __device__ __forceinline__ void step(int warps) { row += warps; settle(); }
 };
 
+// A block's jobs on their way to the job array: a thread's job is 256 bytes, so written by the thread itself
+// each of its 16-byte stores would touch a line of its own.
+constexpr int kJobThreads = 128;
+struct JobStage {
+    uint4 part[kJobThreads][sizeof(TriJob) / 16 + 1];   // a row and 16 bytes: free of bank conflicts
+    __device__ __forceinline__ void put(int t, const TriJob& J) {
+        const uint4* p = reinterpret_cast<const uint4*>(&J);
+#pragma unroll
+        for (int k = 0; k < (int)(sizeof(TriJob) / 16); ++k) part[t][k] = p[k];
+    }
+    // by all threads of the block
+    __device__ __forceinline__ void write(TriJob* __restrict__ jobs, int count) {
+        constexpr int P = sizeof(TriJob) / 16;
+        __syncthreads();
+        for (int i = threadIdx.x; i < count * P; i += kJobThreads) reinterpret_cast<uint4*>(jobs)[i] = part[i / P][i % P];
+    }
+};
+
 __device__ __forceinline__ void sdf_job_prefetch(TriJob* dst, const TriJob* __restrict__ src, int lane) {
     if (lane < (int)(sizeof(TriJob) / 16)) {
         const uint32_t d = (uint32_t)__cvta_generic_to_shared(reinterpret_cast<char*>(dst) + 16 * lane);
