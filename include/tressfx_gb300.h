@@ -339,7 +339,7 @@ int tfx_mesh_read_skinned(tfx_mesh mesh, float* host_dst, size_t bytes);
  * objects at once: skin every collision mesh, rebuild every SDF, run TressFXSimulation::Simulate
  * (TressFXSimulation.cpp:77-112) over every hair object and CollideWithHair
  * (TressFXSDFCollision.cpp:171-221) for each object with its SDF -- as one CUDA-graph launch of a
- * few persistent kernels instead of one dispatch per object per stage.  Results are bit-identical
+ * few kernels instead of one dispatch per object per stage.  Results are bit-identical
  * to the per-object dispatches above.  Objects keep their own buffers (tfx_hair_read / _get_buffer
  * see the batched results); the mesh bound to an SDF must not change after tfx_batch_build. */
 typedef struct tfx_batch_t* tfx_batch;

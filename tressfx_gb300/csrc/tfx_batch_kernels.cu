@@ -2,16 +2,16 @@
 // their SDFs advance one frame in a handful of launches.
 //
 //  * k_batch_mesh_skin    - BoneSkinning (TressFXBoneSkinning.hlsl:57-94) over every vertex of every
-//                           collision mesh.
-//  * k_batch_mesh_skin (its last blocks) / k_batch_sdf_jobs / k_batch_sdf_construct / k_batch_sdf_finalize
-//                         - InitializeSignedDistanceField / ConstructSignedDistanceField /
-//                           FinalizeSignedDistanceField (TressFXSDFCollision.hlsl:301-412) of every
-//                           SDF.  The construct runs one warp per triangle: the lanes share the
-//                           triangle's cell box (the reference's AABB +- one cell, -+ one grid cell),
-//                           the triangle-only terms of the distance are computed once, and each
-//                           (triangle, cell) pair does the reference's distance and an atomicMin on the
-//                           FloatFlip3 word.  The pairs and the encoding are the reference's, so the grid
-//                           is bit-identical.
+//                           collision mesh, and InitializeSignedDistanceField (TressFXSDFCollision.hlsl:
+//                           301-312) of every SDF in its last blocks.
+//  * k_batch_sdf_jobs / k_batch_sdf_construct / k_batch_sdf_finalize
+//                         - ConstructSignedDistanceField / FinalizeSignedDistanceField
+//                           (TressFXSDFCollision.hlsl:329-412) of every SDF.  A thread per triangle
+//                           computes the triangle-only terms and the cell box (the reference's AABB +-
+//                           one cell, -+ one grid cell); the construct's warps run the boxes, leave out the
+//                           cells a lower bound proves the triangle cannot lower, and do the
+//                           reference's distance and an atomicMin on the FloatFlip3 word for the rest.  The
+//                           encoding is the reference's and words only fall, so the grid is bit-identical.
 //  * k_fused_strands      - the six simulation stages of the guide strands (TressFXSimulation.hlsl:
 //                           609-975) for a group of 32 guide strands in one pass.  Phase 0: bulk
 //                           asynchronous copies (cp.async.bulk on an mbarrier) bring the group's Pos
@@ -24,8 +24,8 @@
 //                           exactly the order in which the sequential sweeps read and write).
 //                           Phase 3a (n/VPL lanes per strand): wind, length constraints (warp
 //                           shuffles), tangents, velocity clamp.  Phase 3c: the guides' state is
-//                           written once.  Blocks are persistent over the strand groups of every
-//                           object of one vertices-per-strand class.  Needs no SDF, so it runs
+//                           written once.  A block per strand group of one vertices-per-strand
+//                           class, or persistent blocks over them.  Needs no SDF, so it runs
 //                           while the frame's SDFs are being built.
 //  * k_follow_collide     - UpdateFollowHairVertices (TressFXSimulation.hlsl:978-1001) and the SDF
 //                           collision (TressFXSDFCollision.hlsl:531-595) of every guide and follow
@@ -841,7 +841,7 @@ __device__ __forceinline__ void store_xyz(float4* p, float3 v) {
 // in place of 108) and by how many warps hide them: 64 registers and eight blocks of 128 an SM, at which
 // next to nothing spills once making the follow vertices is a loop of its own.  A thread that made and
 // collided its guide's F + 1 vertices in turn took 80 registers and 112 us a frame of the head, 43.2 of
-// the character (spilling to 64: 124 and 41.0); this form 108.5 and 40.7.  Before the shared corners
+// the character (spilling to 64: 124 and 41.0); this form took 108.5 and 40.7 then.  Before the shared corners
 // (sdf_collide_cell), with per-warp queues of the vertices within the margin: 117 and 41.0; 200,000
 // strands of 16 without follow hairs 283 us, now 259.
 constexpr int kFollowThreads = 128, kFollowBlocksPerSM = 8;
