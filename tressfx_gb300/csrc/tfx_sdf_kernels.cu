@@ -82,7 +82,12 @@ __global__ void __launch_bounds__(256) k_sdf_finalize(uint32_t* __restrict__ sdf
 }
 
 // CollideHairVerticesWithSdf_forward, :531-595.  One thread per hair vertex (guides and follows).
-__global__ void __launch_bounds__(256) k_sdf_collide(const float* __restrict__ sdf, SdfGrid g, float margin,
+//
+// Bound by the gathers and the warps that hide them: 128 threads and ten blocks an SM (48 registers, five
+// words spilled) measured better than 256 threads at 62 registers (a dispatched 6,007 x 64 frame 50.4
+// against 53.0 us, a 2,240 x 32 character 53.4 against 54.1), eight blocks (51.5, 53.7) and twelve (51.4, 54.9).
+constexpr int kCollideThreads = 128;
+__global__ void __launch_bounds__(kCollideThreads, 10) k_sdf_collide(const float* __restrict__ sdf, SdfGrid g, float margin,
                                                      float4* __restrict__ pos, float4* __restrict__ prev,
                                                      int n, long long vtot) {
     after_previous();
@@ -237,7 +242,7 @@ cudaError_t launch_sdf_finalize(uint32_t* sdf, int64_t cells, cudaStream_t s) {
 cudaError_t launch_sdf_collide(const uint32_t* sdf, const SdfGrid& g, float margin, float4* pos, float4* prev, int n,
                                int64_t vtot, cudaStream_t s) {
     if (vtot <= 0) return cudaSuccess;
-    return launch_after(k_sdf_collide, (unsigned)((vtot + 255) / 256), 256, 0, s, reinterpret_cast<const float*>(sdf), g, margin,
+    return launch_after(k_sdf_collide, (unsigned)((vtot + kCollideThreads - 1) / kCollideThreads), kCollideThreads, 0, s, reinterpret_cast<const float*>(sdf), g, margin,
                         pos, prev, n, vtot);
 }
 
