@@ -518,19 +518,24 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1) k_nsdf_train(const __nv_bflo
 }
 
 // Weight and bias gradients, all five layers in one launch: dW_l = H_{l-1}^T dZ_l, db_l = 1^T dZ_l.  A
-// block owns one layer for a part of the batch (`rounds` times 128 samples): it brings both operands into
-// shared memory whole (16-byte copies; rows padded by eight words, which keeps the fragment reads free of
-// bank conflicts), its warps multiply 16-row tiles -- layer 1 has seven of 64 columns, layers 2 to 4 four
-// of which two warps take 32 columns each, layer 5 four of eight -- and it writes its sums to the part's
-// own copy of the gradient, which k_nsdf_adam adds up: the sums do not depend on the order of the blocks.
-// Bound: the latency of the copies.  8,192 samples (ncu): one warp per 16-row tile and 512 samples, added
-// with atomics, 42 us; this split with vector atomics from 64 blocks a word 18 us; as it is 10 us.  32 or 16
-// parts in place of 64 made the whole step slower (21.6 and 26.3 against 20.1 us).
-constexpr int WG_SAMPLES = 128;
+// block owns one layer for a part of the batch (512 samples; `rounds` of them in batches beyond 32,768): it
+// brings both operands into shared memory whole (16-byte copies in four groups; rows padded by eight
+// words, which keeps the fragment reads free of bank conflicts), its warps multiply 16-row tiles -- layer
+// 1 has seven of 64 columns, layers 2 to 4 four of which two warps take 32 columns each, layer 5 four of
+// eight; the bias is one more row of ones -- and it writes its sums to the part's own copy of the gradient,
+// which k_nsdf_adam adds up: the sums do not depend on the order of the blocks.  The tensor cores cut an
+// accumulator off where FP32 addition rounds, so the length of a chain of MMAs shows in the result: 512
+// samples a chain is the length the gradient has always had, and a shorter one (128 samples, 64 parts, 10
+// us) left training off by more than two runs of the atomic form differ.
+// Bound: the latency of the copies and the chain.  8,192 samples (ncu): one warp per 16-row tile and 512
+// samples, added with atomics, took 42 us; a whole step of 8,192 samples takes 19.4 us with this form, 20.1 with
+// 64 parts of 128 samples.
+constexpr int WG_SAMPLES = 512;
 constexpr int WG_PAIRS = WG_SAMPLES / 2;
 constexpr int WG_THREADS = 256;
 constexpr int WG_PAD = 8;
 constexpr size_t WG_SMEM = sizeof(uint32_t) * WG_PAIRS * (KIN + WG_PAD + HID + WG_PAD);
+constexpr int WG_GROUPS = 4;    // copy groups of a part
 constexpr int WG_CHUNK = 512;   // batches are a multiple of this
 
 __global__ void __launch_bounds__(WG_THREADS) k_nsdf_wgrad(const uint32_t* __restrict__ acts, int batch, int rounds,
@@ -554,75 +559,86 @@ __global__ void __launch_bounds__(WG_THREADS) k_nsdf_wgrad(const uint32_t* __res
     const int g = lane >> 2, i = lane & 3;
     after_previous();
     let_next_in();
+    constexpr int GP = WG_PAIRS / WG_GROUPS;
     auto bring = [&](int chunk) {
         const uint32_t* a = Hp + (long long)chunk * WG_PAIRS * fin;
         const uint32_t* b = dZ + (long long)chunk * WG_PAIRS * fout;
-        for (int k = threadIdx.x; k < WG_PAIRS * fin / 4; k += WG_THREADS) {
-            const int r = k / (fin / 4), c = 4 * (k - r * (fin / 4));
-            copy_async16(A + r * sa + c, a + r * fin + c);
+        for (int q = 0; q < WG_GROUPS; ++q) {
+            for (int k = threadIdx.x; k < GP * fin / 4; k += WG_THREADS) {
+                const int r = q * GP + k / (fin / 4), c = 4 * (k % (fin / 4));
+                copy_async16(A + r * sa + c, a + r * fin + c);
+            }
+            for (int k = threadIdx.x; k < GP * fout / 4; k += WG_THREADS) {
+                const int r = q * GP + k / (fout / 4), c = 4 * (k % (fout / 4));
+                copy_async16(B + r * sb + c, b + r * fout + c);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
         }
-        for (int k = threadIdx.x; k < WG_PAIRS * fout / 4; k += WG_THREADS) {
-            const int r = k / (fout / 4), c = 4 * (k - r * (fout / 4));
-            copy_async16(B + r * sb + c, b + r * fout + c);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
+    };
+    auto landed = [&](int q) {   // groups 0 .. q are in shared memory
+        if (q == 0) asm volatile("cp.async.wait_group 3;" ::: "memory");
+        else if (q == 1) asm volatile("cp.async.wait_group 2;" ::: "memory");
+        else if (q == 2) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();
     };
-    // every warp of the block goes through the same rounds; `rows`: it has a tile (mt, columns n0..)
-    auto tile = [&](bool rows, int mt, int n0, auto ntiles) {
+    // every warp of the block goes through the same rounds; `rows`: it has a tile (mt, columns n0..);
+    // `ones`: it has the bias of its columns
+    auto tile = [&](bool rows, bool ones, int mt, int n0, auto ntiles) {
         constexpr int NT = decltype(ntiles)::value;
-        constexpr int BC = 8;   // bias columns of a warp (all 64 of layer 1 over eight warps as well)
-        float C[NT][4], bias[BC];
+        float S[2][NT][4];   // [0] the tile's, [1] the bias's
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) C[nt][q] = 0.f;
-#pragma unroll
-        for (int c = 0; c < BC; ++c) bias[c] = 0.f;
-        const int bc0 = warp * BC;
+            for (int q = 0; q < 4; ++q) S[0][nt][q] = S[1][nt][q] = 0.f;
+        const uint32_t one = g == 0 ? pack_bf16(1.0f, 1.0f) : 0u;
         for (int chunk = chunk0; chunk < chunk1; ++chunk) {
             if (chunk > chunk0) __syncthreads();   // the last round's reads come before its copies
             bring(chunk);
-            if (rows) {
+            float C[2][NT][4];
 #pragma unroll
-                for (int ks = 0; ks < WG_SAMPLES / 16; ++ks) {
-                    const uint32_t* a = A + (8 * ks + i) * sa + mt * 16 + g;   // sample pairs of k rows 2i.. and 2i+8..
-                    const uint32_t* b = B + (8 * ks + i) * sb + n0 + g;
+            for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-                    for (int nt = 0; nt < NT; ++nt)
-                        mma16816(C[nt], a[0], a[8], a[4 * sa], a[4 * sa + 8], b[nt * 8], b[4 * sb + nt * 8]);
+                for (int q = 0; q < 4; ++q) C[0][nt][q] = C[1][nt][q] = 0.f;
+            for (int q = 0; q < WG_GROUPS; ++q) {
+                landed(q);
+#pragma unroll
+                for (int k = 0; k < GP / 8; ++k) {
+                    const int row = q * GP + 8 * k + i;   // sample pairs of k rows 2i.. and 2i+8..
+                    const uint32_t* a = A + row * sa + mt * 16 + g;
+                    const uint32_t* b = B + row * sb + n0 + g;
+                    if (rows)
+#pragma unroll
+                        for (int nt = 0; nt < NT; ++nt)
+                            mma16816(C[0][nt], a[0], a[8], a[4 * sa], a[4 * sa + 8], b[nt * 8], b[4 * sb + nt * 8]);
+                    if (ones)
+#pragma unroll
+                        for (int nt = 0; nt < NT; ++nt) mma16816(C[1][nt], one, 0u, one, 0u, b[nt * 8], b[4 * sb + nt * 8]);
                 }
             }
-            if (bc0 < fout)
 #pragma unroll
-                for (int p = 0; p < WG_PAIRS; p += 32) {
-                    const uint4* b = reinterpret_cast<const uint4*>(B + (p + lane) * sb + bc0);
-                    const uint4 v[2] = {b[0], b[1]};
-                    const uint32_t* u = reinterpret_cast<const uint32_t*>(v);
+            for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-                    for (int c = 0; c < BC; ++c) bias[c] += __uint_as_float(u[c] << 16) + __uint_as_float(u[c] & 0xffff0000u);
-                }
+                for (int q = 0; q < 4; ++q) { S[0][nt][q] += C[0][nt][q]; S[1][nt][q] += C[1][nt][q]; }
         }
         if (rows) {
             float* out = grads + pW + (mt * 16 + g) * fout + n0 + 2 * i;
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
-                *reinterpret_cast<float2*>(out + nt * 8) = make_float2(C[nt][0], C[nt][1]);
-                *reinterpret_cast<float2*>(out + 8 * fout + nt * 8) = make_float2(C[nt][2], C[nt][3]);
+                *reinterpret_cast<float2*>(out + nt * 8) = make_float2(S[0][nt][0], S[0][nt][1]);
+                *reinterpret_cast<float2*>(out + 8 * fout + nt * 8) = make_float2(S[0][nt][2], S[0][nt][3]);
             }
         }
-        if (bc0 < fout)
+        if (ones && g == 0)
 #pragma unroll
-            for (int c = 0; c < BC; ++c) {
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) bias[c] += __shfl_xor_sync(0xffffffffu, bias[c], o);
-                if (lane == 0) grads[pB + bc0 + c] = bias[c];
+            for (int nt = 0; nt < NT; ++nt) {
+                grads[pB + n0 + nt * 8 + 2 * i] = S[1][nt][0];
+                grads[pB + n0 + nt * 8 + 2 * i + 1] = S[1][nt][1];
             }
     };
-    if (layer == 1) tile(warp < KIN / 16, warp, 0, std::integral_constant<int, 8>{});
-    else if (layer < 5) tile(true, warp >> 1, (warp & 1) * 32, std::integral_constant<int, 4>{});
-    else tile(warp < 4, warp, 0, std::integral_constant<int, 1>{});
+    if (layer == 1) tile(warp < KIN / 16, warp == KIN / 16, warp, 0, std::integral_constant<int, 8>{});
+    else if (layer < 5) tile(true, warp < 2, warp >> 1, (warp & 1) * 32, std::integral_constant<int, 4>{});
+    else tile(warp < 4, warp == 4, warp, 0, std::integral_constant<int, 1>{});
 }
 
 // Parameter p's places in the bf16 weight block / bias vector.
@@ -760,7 +776,7 @@ __global__ void k_nsdf_sample(const float4* __restrict__ mesh, int nverts, const
 }  // namespace
 
 // A training step's scratch: the minibatch's activations and gradients in the pair layout, then the parts
-// of the weight gradient (at most TRAIN_PARTS, one per 128 samples or more).
+// of the weight gradient (at most TRAIN_PARTS, one per 512 samples or more).
 constexpr int TRAIN_PARTS = 64;
 static size_t acts_words(int batch) { return (size_t)batch / 2 * (KIN + 8 * HID + OUTN); }
 size_t train_scratch_bytes(int batch) { return 4 * acts_words(batch) + sizeof(float) * (size_t)NPARAM * TRAIN_PARTS; }
