@@ -1,6 +1,6 @@
 """The training step's kernels where their split can go wrong: minibatches of one to several parts of the
-weight gradient, and of more samples than there are parts (two rounds a part, more tiles than the blocks
-take at once), against the NumPy backward pass of the same bf16 network with the bounds of the one-size
+weight gradient, of more tiles than the blocks take at once, and of more samples than there are parts (two
+rounds a part), against the NumPy backward pass of the same bf16 network with the bounds of the one-size
 test; and the same step twice giving the same gradient and weights (its sums do not depend on the order
 of the blocks)."""
 import numpy as np
@@ -14,7 +14,7 @@ BLOCKS = {"W1": (R.P_W1, R.P_B1), "b1": (R.P_B1, R.P_W2), "W2": (R.P_W2, R.P_B2)
           "W5": (R.P_W5, R.P_B5), "b5": (R.P_B5, R.NPARAM)}
 
 
-@pytest.mark.parametrize("batch", [512, 1536, 10240])
+@pytest.mark.parametrize("batch", [512, 1536, 10240, 33280])
 def test_gradient_of_one_step(ctx, batch):
     from tressfx_gb300.api import NeuralSDF
     lo, hi = np.array([-0.2, 1.3, -0.25]), np.array([0.25, 1.8, 0.2])
