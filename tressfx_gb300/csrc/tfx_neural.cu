@@ -688,12 +688,12 @@ __global__ void __launch_bounds__(ADAM_THREADS) k_nsdf_adam(float* __restrict__ 
     const int quad = t >> 3, lane8 = t & 7;
     const bool mine = quad < NPARAM / 4, update = mine && lane8 < 4;
     const int p = 4 * quad + lane8;
-    // written by the step before, which ended before the launches this one follows began
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     const float corr1 = 1.0f - powf(b1, (float)step), corr2 = 1.0f - powf(b2, (float)step);
-    const float m0 = update ? m[p] : 0.f, v0 = update ? v[p] : 0.f, w0 = update ? params[p] : 0.f;
     after_previous();
     let_next_in();
+    // behind the wait: the step before wrote these, and only the wait makes its writes visible here
+    const float m0 = update ? m[p] : 0.f, v0 = update ? v[p] : 0.f, w0 = update ? params[p] : 0.f;
     float4 gr = make_float4(0.f, 0.f, 0.f, 0.f);
     if (mine) {
         const float4* src = reinterpret_cast<const float4*>(parts) + quad;
