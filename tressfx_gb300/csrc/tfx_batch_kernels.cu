@@ -118,9 +118,9 @@ __device__ __forceinline__ int find_by_prefix_tri(const BatchSdf* __restrict__ s
 __device__ __forceinline__ TriJob batch_job(const BatchSdf* __restrict__ sdfs, int nsdf, int t) {
     const BatchSdf& s = sdfs[find_by_prefix_tri(sdfs, nsdf, t)];
     const size_t tri = (size_t)(t - s.firstTriangle);
-    const float3 x0 = xyz(__ldg(s.mesh + 2 * (size_t)__ldg(s.indices + 3 * tri + 0)));
-    const float3 x1 = xyz(__ldg(s.mesh + 2 * (size_t)__ldg(s.indices + 3 * tri + 1)));
-    const float3 x2 = xyz(__ldg(s.mesh + 2 * (size_t)__ldg(s.indices + 3 * tri + 2)));
+    const float3 x0 = xyz(s.mesh[2 * (size_t)__ldg(s.indices + 3 * tri + 0)]);
+    const float3 x1 = xyz(s.mesh[2 * (size_t)__ldg(s.indices + 3 * tri + 1)]);
+    const float3 x2 = xyz(s.mesh[2 * (size_t)__ldg(s.indices + 3 * tri + 2)]);
     return tri_job(s.frame->grid, s.words, x0, x1, x2);
 }
 
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(256) k_batch_sdf_expand(const BatchSdf* __rest
 // ConstructSignedDistanceField, :329-397, over the jobs k_batch_sdf_jobs made (every SDF's triangles in
 // one list).  WARPS = warps per block.
 template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? kConstructBlocksPerSM : 1) k_batch_sdf_construct(const TriJob* __restrict__ jobs, int totalTris) {
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? kConstructBlocksPerSM : 1) k_batch_sdf_construct(const TriJob* jobs, int totalTris) {
     after_previous();
     extern __shared__ __align__(16) unsigned char smem_sdf[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(256, N <= 16 ? 4 : (VPL <= 2 ? 3 : 2)) k_fused
         const WorkItem wi = items[it];
         const BatchObject& ob = objs[wi.obj];
         const HairView h = ob.hair;
-        const DevSimConsts* __restrict__ c = ob.consts;
+        const DevSimConsts* c = ob.consts;
         const int F = h.F;
         const int count = wi.count;
         const int gs0 = wi.firstGuide * (F + 1);   // strand index of the group's first guide
@@ -709,7 +709,7 @@ __global__ void __launch_bounds__(128) k_local_sweep(const BatchObject* __restri
     if (s >= wi.count) return;
     const BatchObject& ob = objs[wi.obj];
     const HairView h = ob.hair;
-    const DevSimConsts* __restrict__ c = ob.consts;
+    const DevSimConsts* c = ob.consts;
     const int iters = c->reserved0;
     if (iters <= 0) return;
     const int gs = (wi.firstGuide + s) * (h.F + 1);
@@ -800,7 +800,7 @@ __device__ __forceinline__ bool follow_group(const BatchObject& ob, FollowGroup&
 
 // A cell's corners from the corner-expanded copy where there is one.
 struct GroupCorners {
-    GridCorners grid;
+    GridCorners<ReadOnlyLoad> grid;
     const float4* sdf8;
     __device__ __forceinline__ void corners(int base, float (&d)[8]) const {
         if (!sdf8) return grid.corners(base, d);
@@ -817,7 +817,7 @@ struct GroupCorners {
 
 // The collision of a vertex at p against the group's SDF.
 __device__ __forceinline__ bool follow_collide_point(const FollowGroup& fg, float3 p, float3& proj) {
-    return sdf_collide_cell(fg.sdf, fg.sg, fg.st, fg.margin, p, proj, GroupCorners{GridCorners(fg.sdf, fg.sg), fg.sdf8});
+    return sdf_collide_cell(fg.sdf, fg.sg, fg.st, fg.margin, p, proj, GroupCorners{GridCorners<ReadOnlyLoad>(fg.sdf, fg.sg), fg.sdf8});
 }
 __device__ __forceinline__ void store_xyz(float4* p, float3 v) {
     *reinterpret_cast<float2*>(p) = make_float2(v.x, v.y);
@@ -1092,7 +1092,7 @@ __global__ void __launch_bounds__(256) k_collide_level(const BatchObject* __rest
         const float* sdf = reinterpret_cast<const float*>(sd.words);
         const float4 hv = h.pos[v];
         float3 proj;
-        if (sdf_collide_point(sdf, g, margin, xyz(hv), proj)) {
+        if (sdf_collide_point<ReadOnlyLoad>(sdf, g, margin, xyz(hv), proj)) {
             h.pos[v] = with_xyz(hv, proj);
             h.prev[v] = with_xyz(h.prev[v], proj);
         }

@@ -118,8 +118,9 @@ __device__ __forceinline__ Q4 quat_from_matrix(const float (&m)[4][4]) {
 
 // Weighted bone blend of ApplyVertexBoneSkinning (matrix path), TressFXSimulation.hlsl:550-566;
 // the same blend is the first half of BoneSkinning, TressFXBoneSkinning.hlsl:67-84.
-// bones: row-major 4x4 matrices, 16 floats each. skin = {boneIndex.xyzw, boneWeight.xyzw}.
-__device__ __forceinline__ void blend_bones(const float4* __restrict__ bones, float4 idx, float4 wgt,
+// bones: row-major 4x4 matrices, 16 floats each, which the launch before may have written: plain loads
+// (tfx_launch.cuh). skin = {boneIndex.xyzw, boneWeight.xyzw}.
+__device__ __forceinline__ void blend_bones(const float4* bones, float4 idx, float4 wgt,
                                             float (&m)[4][4]) {
     const float wv[4] = {wgt.x, wgt.y, wgt.z, wgt.w};
     const float iv[4] = {idx.x, idx.y, idx.z, idx.w};
@@ -127,7 +128,7 @@ __device__ __forceinline__ void blend_bones(const float4* __restrict__ bones, fl
         const float4* M = bones + 4 * ftoi(iv[0]);
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-            float4 row = __ldg(M + r);
+            const float4 row = M[r];
             m[r][0] = row.x * wv[0]; m[r][1] = row.y * wv[0]; m[r][2] = row.z * wv[0]; m[r][3] = row.w * wv[0];
         }
     }
@@ -138,7 +139,7 @@ __device__ __forceinline__ void blend_bones(const float4* __restrict__ bones, fl
             const float4* M = bones + 4 * ftoi(iv[i]);
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
-                float4 row = __ldg(M + r);
+                const float4 row = M[r];
                 m[r][0] = m[r][0] + row.x * wv[i]; m[r][1] = m[r][1] + row.y * wv[i];
                 m[r][2] = m[r][2] + row.z * wv[i]; m[r][3] = m[r][3] + row.w * wv[i];
             }

@@ -356,8 +356,8 @@ __device__ __forceinline__ void bias_quarter(float (&C)[2][4], const float* b, i
     }
 }
 
-__global__ void __launch_bounds__(TRAIN_THREADS, 1) k_nsdf_train(const __nv_bfloat16* __restrict__ wbf,
-                                                                 const float* __restrict__ bias, Frame fr,
+__global__ void __launch_bounds__(TRAIN_THREADS, 1) k_nsdf_train(const __nv_bfloat16* wbf,
+                                                                 const float* bias, Frame fr,
                                                                  const Sample* __restrict__ pool, long long poolSize,
                                                                  int batch, uint32_t seed, uint32_t* __restrict__ acts,
                                                                  float* __restrict__ lossSum) {
@@ -538,7 +538,7 @@ constexpr size_t WG_SMEM = sizeof(uint32_t) * WG_PAIRS * (KIN + WG_PAD + HID + W
 constexpr int WG_GROUPS = 4;    // copy groups of a part
 constexpr int WG_CHUNK = 512;   // batches are a multiple of this
 
-__global__ void __launch_bounds__(WG_THREADS) k_nsdf_wgrad(const uint32_t* __restrict__ acts, int batch, int rounds,
+__global__ void __launch_bounds__(WG_THREADS) k_nsdf_wgrad(const uint32_t* acts, int batch, int rounds,
                                                            float* __restrict__ parts) {
     extern __shared__ uint4 smem_w[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -680,7 +680,7 @@ __global__ void k_nsdf_publish(const float* __restrict__ params, __nv_bfloat16* 
 // four update one parameter each.
 constexpr int ADAM_THREADS = 256;
 static_assert(NPARAM % 4 == 0, "parameters are summed four at a time");
-__global__ void __launch_bounds__(ADAM_THREADS) k_nsdf_adam(float* __restrict__ params, const float* __restrict__ parts, int nparts,
+__global__ void __launch_bounds__(ADAM_THREADS) k_nsdf_adam(float* __restrict__ params, const float* parts, int nparts,
                                                             float* __restrict__ grads, float* __restrict__ m, float* __restrict__ v,
                                                             int step, float lr, __nv_bfloat16* __restrict__ wbf,
                                                             float* __restrict__ bias) {
@@ -996,7 +996,7 @@ __global__ void __launch_bounds__(256) k_band_collide(CollideArgs a) {
         const int v = a.bandList[k];
         const float4 p = a.pos[v];
         float3 proj;
-        if (sdf_collide_point(sdf, a.grid, a.margin, xyz(p), proj)) {
+        if (sdf_collide_point<ReadOnlyLoad>(sdf, a.grid, a.margin, xyz(p), proj)) {
             a.pos[v] = with_xyz(p, proj);
             a.prev[v] = with_xyz(a.prev[v], proj);
         }

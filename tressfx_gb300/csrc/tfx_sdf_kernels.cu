@@ -14,18 +14,18 @@
 namespace tfx {
 
 // --------------------------------------------------------------------------------------------
-__device__ __forceinline__ TriJob plain_job(uint32_t* sdf, const SdfGrid& g, const float4* __restrict__ mesh,
-                                            const uint32_t* __restrict__ idx, int t) {
-    const float3 x0 = xyz(__ldg(mesh + 2 * (size_t)__ldg(idx + 3 * (size_t)t + 0)));
-    const float3 x1 = xyz(__ldg(mesh + 2 * (size_t)__ldg(idx + 3 * (size_t)t + 1)));
-    const float3 x2 = xyz(__ldg(mesh + 2 * (size_t)__ldg(idx + 3 * (size_t)t + 2)));
+__device__ __forceinline__ TriJob plain_job(uint32_t* sdf, const SdfGrid& g, const float4* mesh,
+                                            const uint32_t* idx, int t) {
+    const float3 x0 = xyz(mesh[2 * (size_t)idx[3 * (size_t)t + 0]]);
+    const float3 x1 = xyz(mesh[2 * (size_t)idx[3 * (size_t)t + 1]]);
+    const float3 x2 = xyz(mesh[2 * (size_t)idx[3 * (size_t)t + 2]]);
     return tri_job(g, sdf, x0, x1, x2);
 }
 
 // InitializeSignedDistanceField, :301-312 (vectorised: 4 cells per 16 B store), with the job of every
 // triangle beside it when there is a job array.
 __global__ void __launch_bounds__(256) k_sdf_initialize(uint32_t* __restrict__ sdf, long long cells, SdfGrid g,
-                                                        const float4* __restrict__ mesh, const uint32_t* __restrict__ idx,
+                                                        const float4* mesh, const uint32_t* idx,
                                                         int ntri, TriJob* __restrict__ jobs) {
     after_previous();
     const uint32_t v = float_flip3(1e10f);
@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(256) k_sdf_initialize(uint32_t* __restrict__ s
 }
 
 // ConstructSignedDistanceField, :329-397, over the jobs made beforehand.
-__global__ void __launch_bounds__(128, kConstructBlocksPerSM) k_sdf_construct_jobs(const TriJob* __restrict__ jobs, int ntri) {
+__global__ void __launch_bounds__(128, kConstructBlocksPerSM) k_sdf_construct_jobs(const TriJob* jobs, int ntri) {
     after_previous();
     extern __shared__ __align__(16) unsigned char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -51,8 +51,8 @@ __global__ void __launch_bounds__(128, kConstructBlocksPerSM) k_sdf_construct_jo
 // triangles (sdf_construct_chunk_warp: lane k makes the job of the chunk's k-th triangle), then
 // runs the triangles' cell loops in turn; the warps stride over the chunks.
 __global__ void __launch_bounds__(128) k_sdf_construct(uint32_t* __restrict__ sdf, SdfGrid g,
-                                                       const float4* __restrict__ mesh,
-                                                       const uint32_t* __restrict__ idx, int ntri, int per) {
+                                                       const float4* mesh,
+                                                       const uint32_t* idx, int ntri, int per) {
     after_previous();
     extern __shared__ __align__(16) unsigned char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(256) k_sdf_finalize(uint32_t* __restrict__ sdf
 // words spilled) measured better than 256 threads at 62 registers (a dispatched 6,007 x 64 frame 50.4
 // against 53.0 us, a 2,240 x 32 character 53.4 against 54.1), eight blocks (51.5, 53.7) and twelve (51.4, 54.9).
 constexpr int kCollideThreads = 128;
-__global__ void __launch_bounds__(kCollideThreads, 10) k_sdf_collide(const float* __restrict__ sdf, SdfGrid g, float margin,
+__global__ void __launch_bounds__(kCollideThreads, 10) k_sdf_collide(const float* sdf, SdfGrid g, float margin,
                                                      float4* __restrict__ pos, float4* __restrict__ prev,
                                                      int n, long long vtot) {
     after_previous();
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(kCollideThreads, 10) k_sdf_collide(const float
 // thread per vertex (roots included), one 8-corner fetch, the gradient by forward or backward
 // differences within the same cell (h = 0.1 * cellSize added to the cell-normalised coordinates,
 // as the shader writes it).
-__global__ void __launch_bounds__(256) k_sdf_collide_mixed(const float* __restrict__ sdf, SdfGrid g, float margin,
+__global__ void __launch_bounds__(256) k_sdf_collide_mixed(const float* sdf, SdfGrid g, float margin,
                                                            float4* __restrict__ pos, float4* __restrict__ prev,
                                                            int64_t vtot) {
     after_previous();
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(256) k_sdf_collide_mixed(const float* __restri
     float d[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        d[j] = __ldg(sdf + base + off[j]);
+        d[j] = sdf[base + off[j]];
         if (d[j] == 1e10f) return;
     }
     auto tri = [&](float x, float y, float z) {
@@ -149,15 +149,15 @@ __global__ void __launch_bounds__(256) k_sdf_collide_mixed(const float* __restri
     }
 }
 
-__global__ void __launch_bounds__(256) k_mesh_skin(float4* __restrict__ out, const float4* __restrict__ in,
-                                                   const float4* __restrict__ skin, const float4* __restrict__ bones,
+__global__ void __launch_bounds__(256) k_mesh_skin(float4* __restrict__ out, const float4* in,
+                                                   const float4* skin, const float4* bones,
                                                    int nverts) {
     after_previous();
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nverts) return;
-    const float4 p = __ldg(in + 2 * v), nr = __ldg(in + 2 * v + 1);
+    const float4 p = in[2 * v], nr = in[2 * v + 1];
     float m[4][4];
-    blend_bones(bones, __ldg(skin + 2 * v), __ldg(skin + 2 * v + 1), m);
+    blend_bones(bones, skin[2 * v], skin[2 * v + 1], m);
     out[2 * v] = with_xyz(p, xform_row(xyz(p), 1.0f, m));
     out[2 * v + 1] = with_xyz(nr, xform_row(xyz(nr), 0.0f, m));
 }

@@ -445,14 +445,14 @@ struct JobStage {
     }
 };
 
-__device__ __forceinline__ void sdf_job_prefetch(TriJob* dst, const TriJob* __restrict__ src, int lane) {
+__device__ __forceinline__ void sdf_job_prefetch(TriJob* dst, const TriJob* src, int lane) {
     if (lane < (int)(sizeof(TriJob) / 16)) {
         const uint32_t d = (uint32_t)__cvta_generic_to_shared(reinterpret_cast<char*>(dst) + 16 * lane);
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(reinterpret_cast<const char*>(src) + 16 * lane)
                      : "memory");
     }
 }
-__device__ __forceinline__ void sdf_construct_jobs_warp(const SdfWarpArea& area, const TriJob* __restrict__ jobs, int total,
+__device__ __forceinline__ void sdf_construct_jobs_warp(const SdfWarpArea& area, const TriJob* jobs, int total,
                                                         int warp, int warps, int lane) {
     SdfJobOrder order(total, warp);
     int tri = order.find(warps);
@@ -470,10 +470,11 @@ __device__ __forceinline__ void sdf_construct_jobs_warp(const SdfWarpArea& area,
     }
 }
 
-// GetSignedDistance + TrilinearInterpolate, :414-527
+// GetSignedDistance + TrilinearInterpolate, :414-527.  The grid is what the launch before may have written: plain
+// loads (tfx_launch.cuh).
 __device__ __forceinline__ float lerp_ref(float a, float b, float t) { return a * (1.0f - t) + b * t; }
 
-__device__ __forceinline__ float sdf_lookup(const float* __restrict__ sdf, const SdfGrid& g, float3 p) {
+__device__ __forceinline__ float sdf_lookup(const float* sdf, const SdfGrid& g, float3 p) {
     if (sdf_surely_outside(g, p)) return 1e10f;
     const int3 gc = sdf_coords(g, p);
     if (!(0 <= gc.x && gc.x < g.nx - 2) || !(0 <= gc.y && gc.y < g.ny - 2) || !(0 <= gc.z && gc.z < g.nz - 2))
@@ -481,14 +482,14 @@ __device__ __forceinline__ float sdf_lookup(const float* __restrict__ sdf, const
     const long long X = 1, Y = g.nx, Z = (long long)g.ny * g.nx;
     const long long base = Z * gc.z + Y * gc.y + gc.x;
     float d[8];
-    d[0] = __ldg(sdf + base);
-    d[1] = __ldg(sdf + base + X);
-    d[2] = __ldg(sdf + base + Y);
-    d[3] = __ldg(sdf + base + Y + X);
-    d[4] = __ldg(sdf + base + Z);
-    d[5] = __ldg(sdf + base + Z + X);
-    d[6] = __ldg(sdf + base + Z + Y);
-    d[7] = __ldg(sdf + base + Z + Y + X);
+    d[0] = sdf[base];
+    d[1] = sdf[base + X];
+    d[2] = sdf[base + Y];
+    d[3] = sdf[base + Y + X];
+    d[4] = sdf[base + Z];
+    d[5] = sdf[base + Z + X];
+    d[6] = sdf[base + Z + Y];
+    d[7] = sdf[base + Z + Y + X];
 #pragma unroll
     for (int j = 0; j < 8; ++j)
         if (d[j] == 1e10f) return 1e10f;
@@ -502,7 +503,7 @@ __device__ __forceinline__ float sdf_lookup(const float* __restrict__ sdf, const
 // CollideHairVerticesWithSdf_forward for one vertex (j >= 2): returns true and the projected
 // position when the vertex is pushed out (then Pos.xyz and Prev.xyz both take it).
 // In the shader's own form: the lookup at p and three more, 0.1 cells along each axis.
-static __device__ __noinline__ bool sdf_collide_general(const float* __restrict__ sdf, SdfGrid g, float margin, float3 p, float3* proj) {
+static __device__ __noinline__ bool sdf_collide_general(const float* sdf, SdfGrid g, float margin, float3 p, float3* proj) {
     const float distance = sdf_lookup(sdf, g, p);
     if (distance > margin) return false;
     const float h = 0.1f * g.cell;
@@ -545,7 +546,7 @@ __device__ __forceinline__ bool div_keys(float a, float b, float c) { return min
 // their short form, in place of 27.  corners(base, d) gives the 8 corners of the cell at index base.
 constexpr int kCollideMiss = 0, kCollideHit = 1, kCollideGeneral = 2;
 template <class Corners>
-__device__ __forceinline__ int sdf_collide_shared(const float* __restrict__ sdf, const SdfGrid& g, const SdfSteps& st, float margin,
+__device__ __forceinline__ int sdf_collide_shared(const float* sdf, const SdfGrid& g, const SdfSteps& st, float margin,
                                                  float3 p, float3& proj, const Corners& cell) {
     if (!st.ranged) return kCollideGeneral;
     if (sdf_surely_outside(g, p)) return kCollideMiss;
@@ -603,7 +604,7 @@ __device__ __forceinline__ int sdf_collide_shared(const float* __restrict__ sdf,
 }
 
 template <class Corners>
-__device__ __forceinline__ bool sdf_collide_cell(const float* __restrict__ sdf, const SdfGrid& g, const SdfSteps& st, float margin,
+__device__ __forceinline__ bool sdf_collide_cell(const float* sdf, const SdfGrid& g, const SdfSteps& st, float margin,
                                                  float3 p, float3& proj, const Corners& cell) {
     const int r = sdf_collide_shared(sdf, g, st, margin, p, proj, cell);
     if (r != kCollideGeneral) return r == kCollideHit;
@@ -613,33 +614,45 @@ __device__ __forceinline__ bool sdf_collide_cell(const float* __restrict__ sdf, 
     return true;
 }
 
+// How a kernel reads the finished grid.  PlainLoad anywhere; ReadOnlyLoad only in a kernel launched plainly, which
+// starts when the launches that write the grid have ended (tfx_launch.cuh).
+struct PlainLoad {
+    __device__ __forceinline__ float operator()(const float* p) const { return *p; }
+};
+struct ReadOnlyLoad {
+    __device__ __forceinline__ float operator()(const float* p) const { return __ldg(p); }
+};
+
 // The corners of cell `base` straight from the grid: its own 8, and the 4 that the next cell along an axis adds.
+template <class Load = PlainLoad>
 struct GridCorners {
     const float* sdf;
     int Y, Z;
-    __device__ __forceinline__ GridCorners(const float* __restrict__ s, const SdfGrid& g) : sdf(s), Y(g.nx), Z(g.ny * g.nx) {}
+    __device__ __forceinline__ GridCorners(const float* s, const SdfGrid& g) : sdf(s), Y(g.nx), Z(g.ny * g.nx) {}
     __device__ __forceinline__ float4 four(const float* w, int a, int b, int c, int d) const {
-        return make_float4(__ldg(w + a), __ldg(w + b), __ldg(w + c), __ldg(w + d));
+        const Load load;
+        return make_float4(load(w + a), load(w + b), load(w + c), load(w + d));
     }
     __device__ __forceinline__ void corners(int base, float (&d)[8]) const {
         const float *w00 = sdf + base, *w10 = w00 + Y, *w01 = w00 + Z, *w11 = w01 + Y;
-        d[0] = __ldg(w00);
-        d[1] = __ldg(w00 + 1);
-        d[2] = __ldg(w10);
-        d[3] = __ldg(w10 + 1);
-        d[4] = __ldg(w01);
-        d[5] = __ldg(w01 + 1);
-        d[6] = __ldg(w11);
-        d[7] = __ldg(w11 + 1);
+        const Load load;
+        d[0] = load(w00);
+        d[1] = load(w00 + 1);
+        d[2] = load(w10);
+        d[3] = load(w10 + 1);
+        d[4] = load(w01);
+        d[5] = load(w01 + 1);
+        d[6] = load(w11);
+        d[7] = load(w11 + 1);
     }
     __device__ __forceinline__ float4 beyond_x(int base) const { return four(sdf + base + 2, 0, Y, Z, Z + Y); }
     __device__ __forceinline__ float4 beyond_y(int base) const { return four(sdf + base + 2 * Y, 0, 1, Z, Z + 1); }
     __device__ __forceinline__ float4 beyond_z(int base) const { return four(sdf + base + 2 * Z, 0, 1, Y, Y + 1); }
 };
 
-__device__ __forceinline__ bool sdf_collide_point(const float* __restrict__ sdf, const SdfGrid& g, float margin, float3 p,
-                                                  float3& proj) {
-    return sdf_collide_cell(sdf, g, sdf_steps(g, margin), margin, p, proj, GridCorners(sdf, g));
+template <class Load = PlainLoad>
+__device__ __forceinline__ bool sdf_collide_point(const float* sdf, const SdfGrid& g, float margin, float3 p, float3& proj) {
+    return sdf_collide_cell(sdf, g, sdf_steps(g, margin), margin, p, proj, GridCorners<Load>(sdf, g));
 }
 
 }  // namespace tfx

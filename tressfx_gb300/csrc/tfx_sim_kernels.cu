@@ -22,16 +22,16 @@ namespace tfx {
 template <int N>
 __global__ void __launch_bounds__(256) k_integrate(HairView h) {
     after_previous();
-    const DevSimConsts* __restrict__ c = h.consts;
+    const DevSimConsts* c = h.consts;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= h.G * N) return;
     const int g = t / N, j = t % N;
     const int gs = g * (h.F + 1);
     const int gv = gs * N + j;
 
-    float4 initialPos = __ldg(h.init + gv);
+    float4 initialPos = h.init[gv];
     float m[4][4];
-    blend_bones(c->bones, __ldg(h.skin + 2 * gs), __ldg(h.skin + 2 * gs + 1), m);
+    blend_bones(c->bones, h.skin[2 * gs], h.skin[2 * gs + 1], m);
     const float3 sk = xform_row(xyz(initialPos), 1.0f, m);
     initialPos.x = sk.x; initialPos.y = sk.y; initialPos.z = sk.z;
 
@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(256) k_integrate(HairView h) {
 // CalculateStrandLevelData, TressFXSimulation.hlsl:677-728.  One thread per guide strand.
 __global__ void __launch_bounds__(128) k_strand_level(HairView h) {
     after_previous();
-    const DevSimConsts* __restrict__ c = h.consts;
+    const DevSimConsts* c = h.consts;
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= h.G) return;
     const int gs = g * (h.F + 1);
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(128) k_strand_level(HairView h) {
     if (accel > c->vspAccelThreshold) vspCoeff = 1.0f;
 
     float m[4][4];
-    blend_bones(c->bones, __ldg(h.skin + 2 * gs), __ldg(h.skin + 2 * gs + 1), m);
+    blend_bones(c->bones, h.skin[2 * gs], h.skin[2 * gs + 1], m);
     const Q4 bq = quat_from_matrix(m);
 
     h.sld[3 * gs + 0] = make_float4(bq.x, bq.y, bq.z, bq.w);
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(32) k_local_shape(HairView h) {
     float* BY = BX + N * LD;
     float* BZ = BY + N * LD;                 // [N][LD] bind-pose positions, SoA
 
-    const DevSimConsts* __restrict__ c = h.consts;
+    const DevSimConsts* c = h.consts;
     const int lane = threadIdx.x;
     const int g0 = blockIdx.x * S;
     const int nstr = min(S, h.G - g0);
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(32) k_local_shape(HairView h) {
         P[j * LD + s] = h.pos[gv];
         const float4 bq4 = h.sld[3 * gs];
         const Q4 bq{bq4.x, bq4.y, bq4.z, bq4.w};
-        const float3 b = qrot(bq, xyz(__ldg(h.init + gv)));
+        const float3 b = qrot(bq, xyz(h.init[gv]));
         BX[j * LD + s] = b.x; BY[j * LD + s] = b.y; BZ[j * LD + s] = b.z;
     }
     __syncwarp();
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(256) k_length_wind(HairView h) {
     constexpr int L = N < 32 ? N : 32;
     constexpr int VPL = N / L;
     constexpr int SPW = 32 / L;
-    const DevSimConsts* __restrict__ c = h.consts;
+    const DevSimConsts* c = h.consts;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     const int q = lane % L;
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(256) k_length_wind(HairView h) {
 #pragma unroll
     for (int k = 0; k < VPL; ++k) {
         p[k] = active ? h.pos[base + k] : make_float4(0.f, 0.f, 0.f, 0.f);
-        len[k] = active ? __ldg(h.rest + base + k) : 0.0f;
+        len[k] = active ? h.rest[base + k] : 0.0f;
     }
 
     // ---- wind (all displacements from pre-wind positions)
@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(256) k_length_wind(HairView h) {
 template <int N>
 __global__ void __launch_bounds__(256) k_follow(HairView h) {
     after_previous();
-    const DevSimConsts* __restrict__ c = h.consts;
+    const DevSimConsts* c = h.consts;
     const int per = h.F * N;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= h.G * per) return;
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(256) k_follow(HairView h) {
     const int fv = sbase * N + N + r;
     const float4 p = h.pos[gv];
     const float4 tn = h.tan[gv];
-    const float4 off = __ldg(h.followOffset + sbase + i + 1);
+    const float4 off = h.followOffset[sbase + i + 1];
     const float factor = c->tipSeparation * ((float)j / (float)N) + 1.0f;
     const float4 old = h.pos[fv];
     h.pos[fv] = with_xyz(old, add(xyz(p), mul(factor, xyz(off))));
