@@ -21,7 +21,7 @@ def rate(lr, k, steps):
     return f(lr) * (f(0.1) + f(0.45) * (f(1.0) + c))
 
 
-def network(ctx, pool):
+def network(ctx, pool, weight=1.0):
     from tressfx_gb300.api import NeuralSDF
     lo, hi = np.array([-0.2, 1.3, -0.25]), np.array([0.25, 1.8, 0.2])
     rng = np.random.default_rng(pool)
@@ -29,7 +29,7 @@ def network(ctx, pool):
     samples[:, :3] = rng.uniform(lo, hi, (pool, 3))
     samples[:, 3] = rng.uniform(-3.0, 3.0, pool)
     samples[:, 4:7] = rng.uniform(-0.6, 0.6, (pool, 3))
-    samples[:, 7] = 1.0
+    samples[:, 7] = weight
     nsdf = NeuralSDF(ctx, lo, hi, cell_size=0.004, pose_scale=1.0 / 0.7, seed=29, max_samples=pool, max_eval_samples=0)
     nsdf.set_samples(0, samples)
     return nsdf
@@ -51,3 +51,46 @@ def test_steps_of_one_call_equal_single_steps(ctx, batch, steps):
     for w, g in got[1:]:
         assert np.array_equal(got[0][0], w)
         assert np.array_equal(got[0][1], g)
+
+
+def test_gradient_is_the_rounded_sum_of_its_parts(ctx):
+    """A step's gradient is the sum of one part per 512 samples.  A part by itself is the gradient of the same step
+    with the weight of every other part's samples zero (their terms are exact zeros; samples that two parts draw
+    are left out of both).  The whole gradient is the 64-bit sum of the parts, rounded: parameter by parameter, but
+    for sums within the carried error's own rounding (2^-44 or so) of a rounding boundary, of which 20,000
+    parameters hold none to speak of."""
+    import nsdf_ref as R
+    batch, pool, seed = 4608, 1 << 20, 29
+    drawn = R.drawn_samples(seed, 1, batch, pool).reshape(-1, 512)
+    count = np.zeros(pool, np.int64)
+    for d in drawn:
+        count[np.unique(d)] += 1
+    shared = count > 1
+
+    def gradient(parts):
+        nsdf = network(ctx, pool, weight=np.isin(np.arange(pool), drawn[parts]) & ~shared)
+        nsdf.train(1, batch=batch, lr=1e-3)
+        g = nsdf.gradients()
+        nsdf.close()
+        return g
+
+    exact = sum(gradient([k]).astype(np.float64) for k in range(len(drawn)))
+    whole = gradient(list(range(len(drawn))))
+    assert np.count_nonzero(whole) > 15000
+    assert np.count_nonzero(whole != exact.astype(f)) <= 2
+    ulp = np.spacing(np.abs(whole)).astype(np.float64)
+    assert (np.abs(whole - exact) <= 0.5001 * ulp).all()
+
+
+@pytest.mark.parametrize("batch,digest", [
+    (512, "fd0d026164a943451bef625650d19f591780f039e1bb7506a8ab8f77d0880f3b"),
+    (1024, "5c67298a3a14a3aefa36fdb376ba654a83e692f453d61b351a9fd33e3ee4c3dc")])
+def test_training_of_up_to_two_parts_is_as_ever(ctx, batch, digest):
+    """One part, and two (whose sum has no order), gave the same bits in every run when the parts were added by
+    atomics too: the digest is of that version's weights and gradients after 40 steps."""
+    import hashlib
+    nsdf = network(ctx, 5003)
+    nsdf.train(40, batch=batch, lr=1e-3)
+    h = hashlib.sha256(nsdf.params().tobytes() + nsdf.gradients().tobytes()).hexdigest()
+    nsdf.close()
+    assert h == digest
