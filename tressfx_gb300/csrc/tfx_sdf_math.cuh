@@ -2,6 +2,7 @@
 // collide: FloatFlip3 encoding, grid coordinates, signed point-triangle distance and the
 // trilinear lookup of src/Shaders/TressFXSDFCollision.hlsl, evaluated in the reference's order.
 #pragma once
+#include "tfx_cell_queue.cuh"
 #include "tfx_device_math.cuh"
 #include "tfx_internal.h"
 
@@ -307,7 +308,6 @@ __device__ __forceinline__ void sdf_construct_job_warp(const TriJob& J, uint2* q
     const BoxIndex B = box_index(J.nx, J.nxy, J.inx, J.inxy);
     const float cell = J.cell, R = J.R, slack = J.slack, plane = J.plane, gnx = J.gnx;
     const float bx = J.bx, by = J.by, bz = J.bz, hx = J.hx, hy = J.hy, hz = J.hz, h0 = J.h0;
-    const unsigned below = (1u << lane) - 1u;
     auto word_at = [&](float3 b) { return first + (int)__fmaf_rn(b.z, plane, __fmaf_rn(b.y, gnx, b.x)); };
     // A cell is queued with the word its test read: a distance that is not below it changes nothing (words
     // only fall), and the atomic that would say so is left out.  Atomics are 4 % of the construct: 185 -> 178 us
@@ -319,7 +319,7 @@ __device__ __forceinline__ void sdf_construct_job_warp(const TriJob& J, uint2* q
         const uint32_t w = float_flip3(signed_dist_job(p, J));
         if (w < seen) atomicMin(word_at(b), w);
     };
-    int n = 0;
+    CellQueue<DeviceWarp, uint2*> kept{queue, lane};
     float fc = (float)lane;
     float3 nextCell = box_cell(B, fc);   // each step's word is loaded a step ahead
     uint32_t nextWord = 0u;
@@ -339,23 +339,14 @@ __device__ __forceinline__ void sdf_construct_job_warp(const TriJob& J, uint2* q
         const float cur = __uint_as_float(word >> 1);   // magnitude of the word
         const float thr = __fmaf_rn(cur, 1.0f + 0x1p-15f, slack);
         const bool keep = left > 0 && !(lb2 > __fmul_rn(thr, thr));
-        const unsigned m = __ballot_sync(0xffffffffu, keep);
-        if (keep) queue[n + __popc(m & below)] = make_uint2(__float_as_uint(fc), word);
-        n += __popc(m);
-        if (n >= 32) {
-            __syncwarp();
-            const uint2 e = queue[lane], rest = queue[32 + lane];
-            __syncwarp();
-            queue[lane] = rest;
-            n -= 32;
+        kept.add(keep, make_uint2(__float_as_uint(fc), word));
+        if (kept.full()) {
+            const uint2 e = kept.take();
             evaluate(__uint_as_float(e.x), e.y);
         }
     }
-    __syncwarp();
-    if (lane < n) {
-        const uint2 e = queue[lane];
-        evaluate(__uint_as_float(e.x), e.y);
-    }
+    uint2 e;
+    if (kept.last(e)) evaluate(__uint_as_float(e.x), e.y);
     __syncwarp();
 }
 
