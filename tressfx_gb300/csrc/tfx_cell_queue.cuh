@@ -4,6 +4,9 @@
 //
 // An entry is touched by different lanes from one use to the next, so every such pair of accesses has a sync()
 // between them; a ballot brings the lanes together but orders no memory.
+//
+// What is left after a take moves up: as a ring, with nothing moved but a masked index on every step's entries, a
+// build of 50,040 triangles took 58.3 us, this way 55.5, and a frame of 200,000 strands beside it 286 against 250.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -23,35 +26,37 @@ struct DeviceWarp {
 };
 #endif
 
-// One lane's hold of the queue, a ring.  `entries`: what entries[i] reads and writes.
+// One lane's hold of the queue.  `entries`: what entries[i] reads and writes.
 template <class Warp, class Entries>
 struct CellQueue {
     Entries entries;
     int lane;
-    unsigned head = 0, held = 0;   // the first entry (0 or 32) and how many there are, the same in every lane
+    int n = 0;   // entries held, the same in every lane
 
     // All lanes call it; those with `keep` add `e`.  At most 31 entries are held before it.
     TFX_LANE_FN void add(bool keep, uint2 e) {
         const unsigned m = Warp::ballot(keep);
-        if (keep) entries[(head + held + Warp::count(m & ((1u << lane) - 1u))) & 63u] = e;
-        held += Warp::count(m);
+        if (keep) entries[n + Warp::count(m & ((1u << lane) - 1u))] = e;
+        n += Warp::count(m);
     }
-    TFX_LANE_FN bool full() const { return held >= 32; }
-    // All lanes call it when full(): a lane's own of the first 32 entries.
+    TFX_LANE_FN bool full() const { return n >= 32; }
+    // All lanes call it when full(): a lane's own of the first 32 entries, the others moved up.  Only the live
+    // ones are written: what is added next goes into the entries behind them.
     TFX_LANE_FN uint2 take() {
         Warp::sync();
-        const uint2 e = entries[head + lane];
-        Warp::sync();   // what is added next may go into these entries
-        head ^= 32u;
-        held -= 32;
+        const uint2 e = entries[lane], next = entries[32 + lane];
+        n -= 32;
+        Warp::sync();
+        if (lane < n) entries[lane] = next;
+        Warp::sync();
         return e;
     }
-    // All lanes call it at the end: whether the lane has one of the remaining entries.
+    // All lanes call it at the end: whether the lane has one of the remaining entries.  The caller synchronises
+    // before the entries are used again.
     TFX_LANE_FN bool last(uint2& e) {
         Warp::sync();
-        const bool mine = (unsigned)lane < held;
-        if (mine) e = entries[head + lane];
-        Warp::sync();
+        const bool mine = lane < n;
+        if (mine) e = entries[lane];
         return mine;
     }
 };
