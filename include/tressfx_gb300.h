@@ -250,7 +250,11 @@ int tfx_sdf_create(tfx_context ctx, int64_t alloc_cells, tfx_sdf* out);
 int tfx_sdf_destroy(tfx_sdf sdf);
 /* Binds the collision mesh (TressFXSDFInputMeshInterface::GetMeshBuffer /
  * GetTrimeshVertexIndicesBuffer, TressFXSDFInputMeshInterface.h:38-48): borrowed DEVICE pointers
- * to {float4 position, float4 normal}[num_vertices] and uint32[3*num_triangles]. */
+ * to {float4 position, float4 normal}[num_vertices] and uint32[3*num_triangles].
+ * Device memory: for meshes of 24 triangles an SM (3,648) or more the call takes 256 bytes a triangle as
+ * the build's scratch, so that the builds themselves allocate nothing.  It is kept until the SDF is
+ * destroyed (a recorded build holds its address); a larger mesh takes a further array of at least
+ * twice the size.  Where it cannot be had the call succeeds and builds are slower, with the same result. */
 int tfx_sdf_set_mesh(tfx_sdf sdf, const void* mesh_vertices, int num_vertices, const uint32_t* indices,
                      int num_triangles);
 /* TressFXSDFCollision::Update (TressFXSDFCollision.cpp:95-169): Initialize, Construct, Finalize
@@ -356,7 +360,10 @@ int tfx_batch_add_hair(tfx_batch batch, tfx_hair hair, int sdf_index, int* index
  * hair object in turn (src/Simulation.cpp:106-118).  The hair object must have been added with an
  * SDF, and collides with each SDF once. */
 int tfx_batch_add_hair_collision(tfx_batch batch, int hair_index, int sdf_index);
-/* Builds the object / work / tile tables and captures the frame graphs (reserved must be 0). */
+/* Builds the object / work / tile tables and captures the frame graphs (reserved must be 0).  Among its
+ * device memory are 256 bytes a triangle of all its meshes (from 3,648 triangles on), besides what
+ * tfx_sdf_set_mesh took for each; a batch that cannot have them builds all the same, with the slower
+ * form of the SDF construct. */
 int tfx_batch_build(tfx_batch batch, int reserved);
 /* Times the candidate launch shapes over `frames` frames each on the current inputs, restores every
  * state buffer, and recaptures the graphs with the fastest shapes. */

@@ -864,10 +864,7 @@ extern "C" int tfx_batch_build(tfx_batch b, int reserved) {
     }
     if (nsdf > 0)
         TFX_CUDA(cudaMemcpy(b->sdfTable, sdfs.data(), sizeof(BatchSdf) * nsdf, cudaMemcpyHostToDevice), "tfx_batch: SDFs");
-    if (sdf_takes_jobs(firstTri))
-        TFX_CUDA(cudaMalloc(&b->jobArena, sdf_job_bytes() * (size_t)firstTri), "tfx_batch: triangle jobs");
-    b->sdfL = SdfBatchLaunch{b->sdfTable, nsdf, firstTri, firstQuad, 128, reinterpret_cast<TriJob*>(b->jobArena),
-                             0, nullptr, nullptr, 0, 0};
+    b->sdfL = SdfBatchLaunch{b->sdfTable, nsdf, firstTri, firstQuad, 128, nullptr, 0, nullptr, nullptr, 0, 0};
     if (nsdf > 0) TFX_CUDA(prefer_strand_split(), "tfx_batch: shared-memory split of the SDF kernels");
     b->expandMode = 2;
     if (int r = apply_expand_mode(b)) return r;
@@ -897,6 +894,15 @@ extern "C" int tfx_batch_build(tfx_batch b, int reserved) {
         if (int r = upload_items(c)) return r;
         if (int r = size_class(b, c)) return r;
         b->classes.push_back(std::move(c));
+    }
+    // The construct's job array, the last of the build's allocations so that it takes nothing the others need.  A
+    // batch that cannot have it runs the construct that makes its jobs in shared memory, with the same result.
+    if (sdf_takes_jobs(firstTri)) {
+        if (cudaMalloc(&b->jobArena, sdf_job_bytes() * (size_t)firstTri) != cudaSuccess) {
+            cudaGetLastError();
+            b->jobArena = nullptr;
+        }
+        b->sdfL.jobs = static_cast<TriJob*>(b->jobArena);
     }
     if (int r = capture_graphs(b)) return r;
     b->built = true;
