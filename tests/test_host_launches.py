@@ -68,4 +68,21 @@ def test_batch_builds_without_its_job_array(fake):
     rows = launches()
     assert named(rows, "construct_chunks") and not named(rows, "k_batch_sdf_jobs")
     p.step(0)
+    p.close()
+    """)
+
+
+@pytest.mark.parametrize("triangles,kernel", [(1500, "construct_chunks"), (6000, "k_batch_sdf_construct")])
+def test_sdf_block_is_the_construct_block(fake, triangles, kernel):
+    """TFX_BATCH_SDF_BLOCK is the block size of the construct, with a job array and without."""
+    run(fake, f"""
+    p = batch({triangles})
+    assert named(launches(), "{kernel}") == {{128}}
+    for threads in (64, 256, 128):
+        p.batch.set_option(Batch.SDF_BLOCK, threads)
+        rows = launches()
+        assert named(rows, "{kernel}") == {{threads}}, rows
+        warps = max(b * t // 32 for n, b, t in rows if "{kernel}" in n)
+        assert warps >= {triangles} // 16
+    p.close()
     """)

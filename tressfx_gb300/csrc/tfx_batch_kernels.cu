@@ -201,14 +201,15 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? kConstructBlocksPerSM
 
 // The same without a job array (small batches): each warp takes chunks of `per` consecutive triangles,
 // lane k making the job of the chunk's k-th.
-__global__ void __launch_bounds__(128) k_batch_sdf_construct_chunks(const BatchSdf* __restrict__ sdfs, int nsdf, int totalTris,
-                                                                    int per) {
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) k_batch_sdf_construct_chunks(const BatchSdf* __restrict__ sdfs, int nsdf, int totalTris,
+                                                                           int per) {
     after_previous();
     extern __shared__ __align__(16) unsigned char smem_sdf[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const SdfWarpArea area = sdf_warp_area(smem_sdf, warp, per);
     const int chunks = (totalTris + per - 1) / per;
-    for (int k = blockIdx.x * 4 + warp; k < chunks; k += gridDim.x * 4) {
+    for (int k = blockIdx.x * WARPS + warp; k < chunks; k += gridDim.x * WARPS) {
         const int first = k * per;
         sdf_construct_chunk_warp(area, first, min(per, totalTris - first), lane,
                                  [&](int t) { return batch_job(sdfs, nsdf, t); });
@@ -1131,7 +1132,9 @@ cudaError_t prefer_strand_split() {
     set(k_batch_sdf_construct<2>);
     set(k_batch_sdf_construct<4>);
     set(k_batch_sdf_construct<8>);
-    set(k_batch_sdf_construct_chunks);
+    set(k_batch_sdf_construct_chunks<2>);
+    set(k_batch_sdf_construct_chunks<4>);
+    set(k_batch_sdf_construct_chunks<8>);
     set(k_batch_sdf_finalize);
     set(k_batch_sdf_expand);
     return e;
@@ -1145,8 +1148,8 @@ cudaError_t launch_batch_sdf(const SdfBatchLaunch& L, cudaStream_t s) {
         e = launch_after(k_batch_sdf_jobs, (unsigned)((L.totalTris + kJobThreads - 1) / kJobThreads), kJobThreads, 0, s, L.sdfs, L.nsdf,
                          L.jobs, L.totalTris);
     if (e != cudaSuccess) return e;
+    const int wpb = L.constructThreads / 32;
     if (L.totalTris > 0 && L.jobs) {
-        const int wpb = L.constructThreads / 32;
         const size_t smem = sdf_construct_smem(wpb, kSdfJobsAhead);
         const unsigned blocks = (unsigned)std::min<long long>(((long long)L.totalTris + wpb - 1) / wpb,
                                                               (long long)sm_count() * sdf_construct_blocks_per_sm(L.constructThreads));
@@ -1155,8 +1158,11 @@ cudaError_t launch_batch_sdf(const SdfBatchLaunch& L, cudaStream_t s) {
     } else if (L.totalTris > 0) {
         const int per = sdf_construct_chunk(L.totalTris, sm_count());
         const long long chunks = ((long long)L.totalTris + per - 1) / per;
-        const unsigned blocks = (unsigned)std::min<long long>((chunks + 3) / 4, (long long)sm_count() * 64);
-        e = launch_after(k_batch_sdf_construct_chunks, blocks, 128, sdf_construct_smem(4, per), s, L.sdfs, L.nsdf, L.totalTris, per);
+        const unsigned blocks = (unsigned)std::min<long long>((chunks + wpb - 1) / wpb, (long long)sm_count() * 256 / wpb);
+        e = launch_after(wpb == 2   ? k_batch_sdf_construct_chunks<2>
+                         : wpb == 8 ? k_batch_sdf_construct_chunks<8>
+                                    : k_batch_sdf_construct_chunks<4>,
+                         blocks, 32 * wpb, sdf_construct_smem(wpb, per), s, L.sdfs, L.nsdf, L.totalTris, per);
     }
     if (e == cudaSuccess) e = launch_after(k_batch_sdf_finalize, quad_blocks(q), 256, 0, s, L.sdfs, L.nsdf, q);
     if (e != cudaSuccess || !L.expand) return e;
