@@ -168,7 +168,7 @@ __device__ __forceinline__ DC distance_constraint(float4 p0, float4 p1, float ta
     float3 delta = sub(xyz(p1), xyz(p0));
     const float dd = dot(delta, delta);
     float ratio;   // target / max(|delta|, 1e-7)
-    if (sqrt_inv_in_range<0x28800000u, 0x67800000u>(dd) && fabsf(target) <= 0x1p100f) {
+    if (sqrt_inv_in_range<0x28800000u, 0x67800000u>(dd) && fabsf(target) <= kDivMax) {
         // dd in [2^-46, 2^80]: |delta| is above 1e-7 and in div_by's range; a target below that range gives
         // a ratio far below the last bit of 1, whatever its own last bits
         float s, i;

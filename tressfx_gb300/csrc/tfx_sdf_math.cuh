@@ -208,8 +208,10 @@ __device__ __forceinline__ float edge_dist2_at(float3 p, float3 a, float3 b, flo
 // SignedDistancePointToTriangle of the job's triangle, the bits of signed_dist_pre: the five divisions are
 // by the triangle's own invariants, so they take a multiplication and two fused multiply-adds with the
 // job's reciprocals, and the square root the ranged form; a pair with a numerator below div_by's range (an
-// exact zero among them) or a squared distance outside sqrt_ranged's takes signed_dist_pre.  dot(x2 - p, e)
-// is -dot(p - x2, e): negation is exact and rounding symmetric.
+// exact zero among them) or a squared distance outside sqrt_ranged's takes signed_dist_pre.  Above its range
+// only `na` can lie (a needle: l1 b), and only a quotient beyond the floats would differ: `a` is then NaN
+// where the operator gives an infinity, and either takes the edges.  dot(x2 - p, e) is -dot(p - x2, e):
+// negation is exact and rounding symmetric.
 __device__ __forceinline__ float signed_dist_job(float3 p, const TriJob& J) {
     const float3 x2 = J.x2, px2 = sub(p, x2);
     const float nb = dot(J.x12n, px2);
@@ -587,7 +589,7 @@ __device__ __forceinline__ int sdf_collide_shared(const float* sdf, const SdfGri
     // of zeros has a sign too; a step that spans more than a cell (a cell near p's rounding) shares nothing
     const bool shared = (unsigned)(px - x) <= 1u && (unsigned)(py - y) <= 1u && (unsigned)(pz - z) <= 1u && p.x != 0.0f &&
                         p.y != 0.0f && p.z != 0.0f && distance != 0.0f && div_keys(ax, ay, az) && div_keys(gx, gy, gz) &&
-                        fmaxf(fmaxf(fabsf(gx), fabsf(gy)), fabsf(gz)) <= 0x1p100f;
+                        fmaxf(fmaxf(fabsf(gx), fabsf(gy)), fabsf(gz)) <= kDivMax;
     if (!shared) return kCollideGeneral;
     const float3 nrm = normalize(mk3(div_by(gx, st.h, st.rh), div_by(gy, st.h, st.rh), div_by(gz, st.h, st.rh)));
     proj = add(p, mul(nrm, margin - distance));
