@@ -138,7 +138,12 @@ int tfx_context_create(int device, tfx_context* out);
 int tfx_context_destroy(tfx_context ctx);
 /* Blocks until all work issued on the context's stream has finished (WaitForCompute). */
 int tfx_context_synchronize(tfx_context ctx);
-/* The context's cudaStream_t, as void*. */
+/* The context's cudaStream_t, as void*.  Work of the caller's own may be put on it between the library's
+ * calls, and the calls may be recorded in a stream capture.  The per-object entry points launch their
+ * kernels as programmatic dependent launches: each waits for the work before it by itself, so the order
+ * is the stream's, and a recorded frame holds programmatic edges.  It is instantiated, cloned, nested and
+ * launched as any other; cudaGraphGetEdges and cudaGraphNodeGetDependencies want their edge-data argument
+ * for it (without it they answer cudaErrorLossyQuery). */
 void* tfx_context_stream(tfx_context ctx);
 /* GetTimeStamp(name) (src/EngineInterface.h / DX12EngineInterfaceImpl.cpp:1319-1322): records a
  * named CUDA event on the stream; tfx_context_timestamps returns up to `max` (name, ms since the
