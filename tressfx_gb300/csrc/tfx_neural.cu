@@ -528,8 +528,8 @@ __global__ void __launch_bounds__(TRAIN_THREADS, 1) k_nsdf_train(const __nv_bflo
 // samples a chain is the length the gradient has always had, and a shorter one (128 samples, 64 parts, 10
 // us) left training off by more than two runs of the atomic form differ.
 // Bound: the latency of the copies and the chain.  8,192 samples (ncu): one warp per 16-row tile and 512
-// samples, added with atomics, took 42 us; a whole step of 8,192 samples takes 19.4 us with this form, 20.1 with
-// 64 parts of 128 samples.
+// samples, added with atomics, took 42 us, this form 11; a whole step of 8,192 samples took 19.4 us with it when 64 parts of
+// 128 samples took 20.1.
 constexpr int WG_SAMPLES = 512;
 constexpr int WG_PAIRS = WG_SAMPLES / 2;
 constexpr int WG_THREADS = 256;
@@ -685,16 +685,18 @@ struct CarrySum {
         rest += ((sum - (s - b)) + (x - b)) + r;
         sum = s;
     }
+    __device__ __forceinline__ void add(const CarrySum& x) { add(x.sum, x.rest); }
     __device__ __forceinline__ float value() const { return sum + rest; }
 };
 
 // The gradient as the sum of its `nparts` parts, Adam (Kingma & Ba 2015) on the fp32 master parameters, then
-// their copies.  Eight lanes share four consecutive parameters: each adds an eighth of the parts, the first
-// four update one parameter each.  The parts were once added by atomics in the order in which blocks ended, and
+// their copies.  Eight lanes share four consecutive parameters: each adds an eighth of the parts, every other
+// lane updates one parameter.  The parts were once added by atomics in the order in which blocks ended, and
 // every order rounds differently: training follows such a difference (a weight at a bf16 boundary flips, and the
 // gradients part by 1e-5 to 1e-3 within 64 steps).  The exact sum is the middle of what the orders give:
 // after 40 steps of 4,608 samples its gradients are at 6e-8 from a run with atomics in the median, where two such
-// runs are at 2e-5 (and a fixed tree of FP32 additions was at 1e-5).
+// runs are at 2e-5 (and a fixed tree of FP32 additions was at 1e-5).  It costs 0.3 us of a step's 19.8 (8,192
+// samples).
 constexpr int ADAM_THREADS = 256;
 static_assert(NPARAM % 4 == 0, "parameters are summed four at a time");
 __global__ void __launch_bounds__(ADAM_THREADS) k_nsdf_adam(float* __restrict__ params, const float* parts, int nparts,
@@ -703,8 +705,8 @@ __global__ void __launch_bounds__(ADAM_THREADS) k_nsdf_adam(float* __restrict__ 
                                                             float* __restrict__ bias) {
     const int t = blockIdx.x * ADAM_THREADS + threadIdx.x;
     const int quad = t >> 3, lane8 = t & 7;
-    const bool mine = quad < NPARAM / 4, update = mine && lane8 < 4;
-    const int p = 4 * quad + lane8;
+    const bool mine = quad < NPARAM / 4, update = mine && (lane8 & 1) == 0;
+    const int p = 4 * quad + (lane8 >> 1);
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     const float corr1 = 1.0f - powf(b1, (float)step), corr2 = 1.0f - powf(b2, (float)step);
     after_previous();
@@ -720,12 +722,19 @@ __global__ void __launch_bounds__(ADAM_THREADS) k_nsdf_adam(float* __restrict__ 
             gr[0].add(x.x); gr[1].add(x.y); gr[2].add(x.z); gr[3].add(x.w);
         }
     }
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1) gr[k].add(__shfl_xor_sync(0xffffffffu, gr[k].sum, o), __shfl_xor_sync(0xffffffffu, gr[k].rest, o));
+    // the eight lanes' sums: a lane gives away two of its four parameters, then one of two, then adds its neighbour's
+    auto from = [](const CarrySum& x, int o) {
+        return CarrySum{__shfl_xor_sync(0xffffffffu, x.sum, o), __shfl_xor_sync(0xffffffffu, x.rest, o)};
+    };
+    const bool upper = lane8 & 4, odd = lane8 & 2;
+    CarrySum pair[2] = {upper ? gr[2] : gr[0], upper ? gr[3] : gr[1]};
+    pair[0].add(from(upper ? gr[0] : gr[2], 4));
+    pair[1].add(from(upper ? gr[1] : gr[3], 4));
+    CarrySum all = odd ? pair[1] : pair[0];
+    all.add(from(odd ? pair[0] : pair[1], 2));
+    all.add(from(all, 1));
     if (!update) return;
-    const float g = lane8 == 0 ? gr[0].value() : lane8 == 1 ? gr[1].value() : lane8 == 2 ? gr[2].value() : gr[3].value();
+    const float g = all.value();
     grads[p] = g;
     const float mm = b1 * m0 + (1.0f - b1) * g;
     const float vv = b2 * v0 + (1.0f - b2) * g * g;
