@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? kConstructBlocksPerSM
 // lane k making the job of the chunk's k-th.
 template <int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) k_batch_sdf_construct_chunks(const BatchSdf* __restrict__ sdfs, int nsdf, int totalTris,
-                                                                           int per) {
+                                                                           int per, bool all) {
     after_previous();
     extern __shared__ __align__(16) unsigned char smem_sdf[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_batch_sdf_construct_chunks(const
     const int chunks = (totalTris + per - 1) / per;
     for (int k = blockIdx.x * WARPS + warp; k < chunks; k += gridDim.x * WARPS) {
         const int first = k * per;
-        sdf_construct_chunk_warp(area, first, min(per, totalTris - first), lane,
+        sdf_construct_chunk_warp(area, first, min(per, totalTris - first), lane, all,
                                  [&](int t) { return batch_job(sdfs, nsdf, t); });
     }
 }
@@ -1162,7 +1162,8 @@ cudaError_t launch_batch_sdf(const SdfBatchLaunch& L, cudaStream_t s) {
         e = launch_after(wpb == 2   ? k_batch_sdf_construct_chunks<2>
                          : wpb == 8 ? k_batch_sdf_construct_chunks<8>
                                     : k_batch_sdf_construct_chunks<4>,
-                         blocks, 32 * wpb, sdf_construct_smem(wpb, per), s, L.sdfs, L.nsdf, L.totalTris, per);
+                         blocks, 32 * wpb, sdf_construct_smem(wpb, per), s, L.sdfs, L.nsdf, L.totalTris, per,
+                         !sdf_fills_device(L.totalTris, sm_count()));
     }
     if (e == cudaSuccess) e = launch_after(k_batch_sdf_finalize, quad_blocks(q), 256, 0, s, L.sdfs, L.nsdf, q);
     if (e != cudaSuccess || !L.expand) return e;

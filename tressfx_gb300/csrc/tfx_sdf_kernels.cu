@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(128, kConstructBlocksPerSM) k_sdf_construct_jo
 // runs the triangles' cell loops in turn; the warps stride over the chunks.
 __global__ void __launch_bounds__(128) k_sdf_construct(uint32_t* __restrict__ sdf, SdfGrid g,
                                                        const float4* mesh,
-                                                       const uint32_t* idx, int ntri, int per) {
+                                                       const uint32_t* idx, int ntri, int per, bool all) {
     after_previous();
     extern __shared__ __align__(16) unsigned char smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(128) k_sdf_construct(uint32_t* __restrict__ sd
     const int chunks = (ntri + per - 1) / per;
     for (int k = blockIdx.x * (blockDim.x >> 5) + warp; k < chunks; k += warpsTotal) {
         const int first = k * per;
-        sdf_construct_chunk_warp(area, first, min(per, ntri - first), lane, [&](int t) {
+        sdf_construct_chunk_warp(area, first, min(per, ntri - first), lane, all, [&](int t) {
             return plain_job(sdf, g, mesh, idx, t);
         });
     }
@@ -195,7 +195,7 @@ static inline unsigned grid_for(long long work, int threads, unsigned cap) {
 }
 
 size_t sdf_job_bytes() { return sizeof(TriJob); }
-bool sdf_takes_jobs(int64_t tris) { return sdf_wants_jobs(tris, sm_count()); }
+bool sdf_takes_jobs(int64_t tris) { return sdf_fills_device(tris, sm_count()); }
 
 cudaError_t launch_upload(void* dst, const void* pinned, size_t bytes, cudaStream_t s) {
     const int quads = (int)(bytes / 16);
@@ -231,7 +231,8 @@ cudaError_t launch_sdf_construct(uint32_t* sdf, const SdfGrid& g, const float4* 
     const int per = sdf_construct_chunk(ntri, sm_count());
     const long long chunks = ((long long)ntri + per - 1) / per;
     const unsigned blocks = (unsigned)std::min<long long>((chunks + 3) / 4, (long long)sm_count() * 64);
-    return launch_after(k_sdf_construct, blocks, 128, sdf_construct_smem(4, per), s, sdf, g, mesh, idx, ntri, per);
+    return launch_after(k_sdf_construct, blocks, 128, sdf_construct_smem(4, per), s, sdf, g, mesh, idx, ntri, per,
+                        !sdf_fills_device(ntri, sm_count()));
 }
 
 cudaError_t launch_sdf_finalize(uint32_t* sdf, int64_t cells, cudaStream_t s) {

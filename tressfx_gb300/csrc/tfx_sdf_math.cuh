@@ -205,13 +205,21 @@ __device__ __forceinline__ float edge_dist2_at(float3 p, float3 a, float3 b, flo
     return dot(q, q);
 }
 
+// A key of a numerator that is below kNumKey exactly where the numerator is below div_by's range and not zero (twice
+// the bits less one, which makes a zero of either sign the largest).
+__device__ __forceinline__ uint32_t num_key(float a) { return 2u * __float_as_uint(a) - 1u; }
+constexpr uint32_t kNumKey = 2u * 0x21800000u - 1u;   // kDivMin's
+
 // SignedDistancePointToTriangle of the job's triangle, the bits of signed_dist_pre: the five divisions are
 // by the triangle's own invariants, so they take a multiplication and two fused multiply-adds with the
-// job's reciprocals, and the square root the ranged form; a pair with a numerator below div_by's range (an
-// exact zero among them) or a squared distance outside sqrt_ranged's takes signed_dist_pre.  Above its range
-// only `na` can lie (a needle: l1 b), and only a quotient beyond the floats would differ: `a` is then NaN
-// where the operator gives an infinity, and either takes the edges.  dot(x2 - p, e) is -dot(p - x2, e):
-// negation is exact and rounding symmetric.
+// job's reciprocals, and the square root the ranged form; a pair with a numerator below div_by's range or a
+// squared distance outside sqrt_ranged's takes signed_dist_pre.  A numerator of exactly zero, which whole planes
+// of cells have around an axis-aligned mesh, is fine: its quotient may come out as the other zero, which no
+// comparison, clamp or square tells apart.  (Sent to signed_dist_pre as well, zeros made a box of 48 triangles in
+// 128^3 take 192 us, 82 without; before the short forms it was 151.)  Above the range only `na` can lie (a
+// needle: l1 b), and only a quotient beyond the floats would differ: `a` is then NaN where the operator gives an
+// infinity, and either takes the edges.  dot(x2 - p, e) is -dot(p - x2, e): negation is exact and rounding
+// symmetric.
 __device__ __forceinline__ float signed_dist_job(float3 p, const TriJob& J) {
     const float3 x2 = J.x2, px2 = sub(p, x2);
     const float nb = dot(J.x12n, px2);
@@ -221,20 +229,22 @@ __device__ __forceinline__ float signed_dist_job(float3 p, const TriJob& J) {
     const float c = (1.0f - a) - b;
     const float tol = 1e-8f;
     const float3 x0 = J.x0, x1 = J.x1;
-    float least = fminf(fabsf(na), fabsf(nb));
+    uint32_t least = min(num_key(na), num_key(nb));
     float d2;
     if (a >= -tol && b >= -tol && c >= -tol) {
         const float3 nn = sub(p, add(add(mul(a, x0), mul(b, x1)), mul(c, x2)));
         d2 = dot(nn, nn);
     } else {
         const float n01 = dot(sub(x1, p), J.e01), n12 = -dot(px2, J.e12), n02 = -dot(px2, sub(x2, x0));
-        least = fminf(fminf(least, fabsf(n01)), fminf(fabsf(n12), fabsf(n02)));
+        least = min(least, num_key(n01));
+        least = min(least, num_key(n12));
+        least = min(least, num_key(n02));
         const float u01 = edge_dist2_at(p, x0, x1, div_by(n01, J.d01, J.r01));
         const float u12 = edge_dist2_at(p, x1, x2, div_by(n12, J.d12, J.r12));
         const float u02 = edge_dist2_at(p, x0, x2, div_by(n02, J.d02, J.r02));
         d2 = fminf(fminf(u01, u12), u02);
     }
-    if (!J.ranged || !(least >= kDivMin) || !sqrt_in_range(d2)) return signed_dist_pre(p, job_pre(J));
+    if (!J.ranged || least < kNumKey || !sqrt_in_range(d2)) return signed_dist_pre(p, job_pre(J));
     const float d = sqrt_ranged(d2);
     return (dot(sub(p, x0), J.nTri) < 0.0f) ? -d : d;
 }
@@ -285,13 +295,16 @@ __device__ __forceinline__ float3 box_cell(const BoxIndex& B, float c) {
 // sqrt(2) times the bound plus R.  All are well inside the slack: 2^-17 of max|x_i| + |origin| + box + R + w
 // and 2^-15 of the word itself.  A NaN keeps the cell.
 //
-// A box that is not narrow has every cell evaluated.
+// A box that is not narrow has every cell evaluated, and so has every box of a launch too small to fill the device
+// (`all`): there a triangle's time is its one warp's chain, which the tests lengthen, and few words are low enough
+// to decide one.  A 12-triangle box in 64^3: 106 us with the tests, 75 without (115 before there were any); 816
+// triangles in 128^3: 52 and 43 (55); 3,474 in 64^3: 17.5 and 16.2 (25).
 //
 // Bound: issue, and the latency of a step's chain (26 warps per SM).  About 50 instructions test 32 cells,
 // about 230 evaluate 32; of the 200 cells of a box 35 are evaluated, in 1.6 steps of 6.6.  50,040
 // triangles on a 128^3 grid: 42 M warp instructions and 58 us (ncu), where evaluating every cell took
 // 96 M and 97 us.  Each step loads its words one step ahead (61 us without).
-__device__ __forceinline__ void sdf_construct_job_warp(const TriJob& J, uint2* queue, int lane) {
+__device__ __forceinline__ void sdf_construct_job_warp(const TriJob& J, uint2* queue, int lane, bool all) {
     const int vol = J.vol;
     uint32_t* const first = J.first;
     if (!J.narrow) {
@@ -321,6 +334,11 @@ __device__ __forceinline__ void sdf_construct_job_warp(const TriJob& J, uint2* q
         const uint32_t w = float_flip3(signed_dist_job(p, J));
         if (w < seen) atomicMin(word_at(b), w);
     };
+    if (all) {
+        for (int c = lane; c < vol; c += 32) evaluate((float)c, 0xffffffffu);
+        __syncwarp();
+        return;
+    }
     CellQueue<DeviceWarp, uint2*> kept{queue, lane};
     float fc = (float)lane;
     float3 nextCell = box_cell(B, fc);   // each step's word is loaded a step ahead
@@ -376,25 +394,30 @@ inline int sdf_construct_chunk(long long tris, int sms) {
     const long long per = tris / ((long long)sms * 24);
     return (int)(per < 1 ? 1 : per > 16 ? 16 : per);
 }
-// Whether a launch over `tris` triangles takes its jobs from a job array.  Below one triangle per resident
-// warp, making the jobs beside the words' initialisation only lengthens the initialisation: a whole build
-// of 1,486 / 3,016 / 4,468 / 25,700 triangles takes 20.5 / 22.8 / 25.6 / 45.1 us with the array, 18.9 /
-// 22.5 / 26.6 / 56.8 us with each warp making its own.
-inline bool sdf_wants_jobs(long long tris, int sms) { return tris >= (long long)sms * 24; }
+// Whether a launch over `tris` triangles fills the device: a triangle for every resident warp.  From there on the
+// construct reads its jobs from an array, where it has one, and tests the cells; below, its warps make their own
+// and evaluate every cell (sdf_construct_job_warp).  Around the line the two ways to the jobs are equal: a plain
+// rebuild in 64^3 of 2,500 / 3,600 / 4,500 / 6,000 / 9,000 triangles takes 13.8 / 14.0 / 13.9 / 14.2 / 16.2 us
+// with the array, 14.2 / 14.2 / 14.4 / 16.1 / 17.0 with each warp making its own; a batched frame of 2,240 x 32
+// strands around it 21.3 / 22.3 / 22.7 / 23.9 / 26.0 and 21.4 / 22.8 / 22.9 / 25.0 / 26.9.  Well above it, the
+// array is ahead where the strand kernels fill the device (200,000 x 16 and 50,000 triangles: 251 against 283 us)
+// and behind where a frame is little else than its mesh (2,240 x 32 and 25,800: 40.3 against 37.2).
+inline bool sdf_fills_device(long long tris, int sms) { return tris >= (long long)sms * 24; }
 
 // One warp's chunk of `count` (<= the area's jobs) consecutive triangles starting at `first`: lane k makes
 // the job of triangle first + k with make(t), then the warp runs the cell loops; the chunk ends with the
 // warp synchronised, so the area can take the next chunk.
 template <class MakeJob>
-__device__ __forceinline__ void sdf_construct_chunk_warp(const SdfWarpArea& area, int first, int count, int lane, MakeJob make) {
+__device__ __forceinline__ void sdf_construct_chunk_warp(const SdfWarpArea& area, int first, int count, int lane, bool all,
+                                                         MakeJob make) {
     if (lane < count) area.jobs[lane] = make(first + lane);
     __syncwarp();
-    for (int j = 0; j < count; ++j) sdf_construct_job_warp(area.jobs[j], area.queue, lane);
+    for (int j = 0; j < count; ++j) sdf_construct_job_warp(area.jobs[j], area.queue, lane, all);
     __syncwarp();
 }
 
-// The construct over an array of jobs made beforehand (a thread per triangle, beside the words'
-// initialisation): the launch's warps stride over the triangles, each bringing its next job into shared
+// The construct over an array of jobs made beforehand (a thread per triangle: beside the words' initialisation on
+// the plain path, in a launch of its own in a batch): the launch's warps stride over the triangles, each bringing its next job into shared
 // memory while it runs the current one.  Triangles are taken 16 apart, the starting points in
 // bit-reversed order, so that the first ones already give every part of the mesh a word near its result
 // and the later ones find most of their cells decided.
@@ -459,7 +482,7 @@ __device__ __forceinline__ void sdf_construct_jobs_warp(const SdfWarpArea& area,
         asm volatile("cp.async.commit_group;" ::: "memory");
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncwarp();
-        sdf_construct_job_warp(area.jobs[cur], area.queue, lane);   // ends with the warp synchronised
+        sdf_construct_job_warp(area.jobs[cur], area.queue, lane, false);   // ends with the warp synchronised
     }
 }
 
