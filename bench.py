@@ -66,13 +66,13 @@ WORKLOADS = {
 # profiles/).  ncu flushes the caches before the capture and does not count writes still in L2 when
 # the kernel ends.  These are recorded figures, not measured by this run.
 NCU_TRAFFIC = {
-    ("head", "k_follow_collide (n=32)"): 105.3e6,
-    ("head", "k_fused_strands (n=32)"): 48.3e6,
-    # captured on the first 8 objects (5.54 M of the class's 18.69 M vertices, 784.6 MB; the kernel
+    ("head", "k_follow_collide (n=32)"): 96.2e6,
+    ("head", "k_fused_strands (n=32)"): 48.4e6,
+    # captured on the first 8 objects (5.54 M of the class's 18.69 M vertices, 781.4 MB; the kernel
     # streams each vertex's rows a fixed number of times, so traffic grows with the vertices): scaled
     # to the full launch
-    ("batched", "k_fused_strands (n=64)"): 2647.0e6,
-    ("fur", "k_fused_strands (n=16)"): 387.8e6,
+    ("batched", "k_fused_strands (n=64)"): 2636.2e6,
+    ("fur", "k_fused_strands (n=16)"): 382.1e6,
 }
 
 
