@@ -45,8 +45,8 @@ def batch(triangles):
 """
 
 
-def run(fake, code):
-    env = dict(os.environ, PYTHONPATH=str(ROOT))
+def run(fake, code, **more):
+    env = dict(os.environ, PYTHONPATH=str(ROOT), **more)
     r = subprocess.run([sys.executable, "-c", PRELUDE + textwrap.dedent(code), str(fake)], env=env, capture_output=True, text=True,
                        timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
@@ -86,3 +86,14 @@ def test_sdf_block_is_the_construct_block(fake, triangles, kernel):
         assert warps >= {triangles} // 16
     p.close()
     """)
+
+
+def test_objects_may_go_before_the_batch(fake):
+    """Destroying a batch reads nothing of the objects that it held, which a program may have destroyed before it
+    (freed memory is overwritten here, so that reading it shows)."""
+    run(fake, """
+    p = batch(1500)
+    for x in p.hair + p.sdfs + p.meshes:
+        x.close()
+    p.batch.close()
+    """, MALLOC_PERTURB_="165", GLIBC_TUNABLES="glibc.malloc.tcache_count=0")

@@ -184,10 +184,10 @@ extern "C" int tfx_batch_destroy(tfx_batch b) {
         if (t) cudaFree(t);
     for (auto& c : b->classes)
         if (c.items) cudaFree(c.items);
-    for (auto h : b->hairs) context_release(h->ctx);
-    for (auto s : b->sdfs) context_release(s->ctx);
-    for (auto m : b->sdfMesh)
-        if (m) context_release(m->ctx);
+    // a reference for each object added, all of this context; the objects themselves may be gone
+    size_t refs = b->hairs.size() + b->sdfs.size();
+    for (auto m : b->sdfMesh) refs += m != nullptr;
+    for (; refs > 0; --refs) context_release(b->ctx);
     context_release(b->ctx);
     delete b;
     return TFX_OK;
